@@ -14,6 +14,7 @@
 
 #include "r2d3c_aux.cuh"
 #include "r2d3c_engine.h"
+#include "r2d3c_pass64.cuh"
 
 namespace r2d3c {
 
@@ -108,6 +109,14 @@ class EngineT final : public IEngine {
       enc_base_ = enc_ = alloc<unsigned long long>((size_t)kScalStride * nb_);
       d_sc_ = alloc<StepCoef>(nb_);
       d_cfl_ = alloc<CflCoef>(nb_);
+      if (full && sizeof(T) == 8) {  // pass C's tables (RkTab)
+        const size_t w = (size_t)gd_.L + 1;
+        rk_run_ = (size_t)gd_.M * w;
+        rk_d1_ = alloc<double>(rk_run_ * nb_);
+        rk_d2_ = alloc<double>(rk_run_ * nb_);
+        rk_ik2_ = alloc<double>(rk_run_);
+        rk_wk_ = alloc<double>(w * nb_);
+      }
       dirty_.assign(nb_, 0);
       partials_ = alloc<double>((size_t)kSumBlocks * kMaxTerms);
       small_ = alloc<double>((size_t)kMaxTerms + 5 * (size_t)gd_.nh);
@@ -778,6 +787,7 @@ class EngineT final : public IEngine {
   // per-run coefficient arrays: nb == 1 takes mc, a batch its run coefficients
   // (skipped when the device already holds the same coefficients: a caller
   // that advances one step per call pays no copy and no synchronisation)
+  // FP64: new step coefficients rebuild pass C's tables on the engine stream.
   void upload_coefs(const ModelCoef& mc, double cfl) {
     if (nb_ == 1) coefs_.assign(1, mc);
     if ((int)coefs_.size() != nb_) throw Error(kESTATE, "run coefficients not set");
@@ -789,15 +799,22 @@ class EngineT final : public IEngine {
       cc[r] = cfl_coef(cfl, m);
     }
     const size_t bs = sizeof(StepCoef) * nb_, bc = sizeof(CflCoef) * nb_;
-    if (coefs_valid_ && up_sc_.size() == bs && up_cc_.size() == bc && std::memcmp(up_sc_.data(), sc.data(), bs) == 0 &&
-        std::memcmp(up_cc_.data(), cc.data(), bc) == 0)
-      return;
+    const bool same_sc = sc_valid_ && up_sc_.size() == bs && std::memcmp(up_sc_.data(), sc.data(), bs) == 0;
+    if (coefs_valid_ && same_sc && up_cc_.size() == bc && std::memcmp(up_cc_.data(), cc.data(), bc) == 0) return;
     cuda_check(cudaMemcpyAsync(d_sc_, sc.data(), bs, cudaMemcpyHostToDevice, st_), "H2D step coefs");
     cuda_check(cudaMemcpyAsync(d_cfl_, cc.data(), bc, cudaMemcpyHostToDevice, st_), "H2D cfl coefs");
+    if (!same_sc) build_rk_tables();
     sync();
+    sc_valid_ = true;
     up_sc_.assign(reinterpret_cast<const char*>(sc.data()), reinterpret_cast<const char*>(sc.data()) + bs);
     up_cc_.assign(reinterpret_cast<const char*>(cc.data()), reinterpret_cast<const char*>(cc.data()) + bc);
     coefs_valid_ = true;
+  }
+
+  void build_rk_tables() {
+    if (!rk_d1_) return;
+    k_rk_table<<<dim3(elem_blocks(rk_run_), nb_), 256, 0, st_>>>(rk_d1_, rk_d2_, rk_ik2_, rk_wk_, gd_, d_sc_);
+    post("k_rk_table");
   }
 
   template <typename U>
@@ -1024,7 +1041,7 @@ class EngineT final : public IEngine {
   void launch_colfft_mixed(const cpx<T>* in, cpx<T>* out) {
     dispatch_n(n_, [&](auto NC) {
       constexpr int N = decltype(NC)::value;
-      constexpr int PY = PassNT<T, N>::value;
+      constexpr int PY = sizeof(T) == 8 ? 2 : PassNT<T, N>::value;
       using C = Cfg<T, N>;
       auto k = k_colfft<T, N, -1, PY>;
       const int g = fft_groups(gd_.nh, C::G);
@@ -1056,6 +1073,20 @@ class EngineT final : public IEngine {
   }
   Batch batch() const { return Batch{S_, (size_t)6 * gd_.M * n_, 2 * S_}; }
   void launch_passA(const cpx<T>* a, const cpx<T>* b, cpx<T>* tf, int nb) {
+    if constexpr (sizeof(T) == 8) launch_passA64(a, b, tf, nb);
+    else launch_passA32(a, b, tf, nb);
+  }
+  void launch_passA64(const cpx<T>* a, const cpx<T>* b, cpx<T>* tf, int nb) {
+    dispatch_n(n_, [&](auto NC) {
+      constexpr int N = decltype(NC)::value;
+      using C = Cfg<T, N>;
+      const int g = ga_ ? ga_ : C::G;  // groups per CTA, field chunks: autotuned
+      const dim3 grid((gd_.M + g - 1) / g, nb, fa_);
+      k_passA64<N><<<grid, C::TPF * g, g * C::FFT::SMEM_BYTES, st_>>>(a, b, tf, gd_, tw_, batch());
+      post("k_passA64");
+    });
+  }
+  void launch_passA32(const cpx<T>* a, const cpx<T>* b, cpx<T>* tf, int nb) {
     dispatch_n(n_, [&](auto NC) {
       constexpr int N = decltype(NC)::value;
       constexpr int NT = PassNT<T, N>::value;
@@ -1080,8 +1111,35 @@ class EngineT final : public IEngine {
       go(std::integral_constant<int, PassAE<T, N>::value>{});
     });
   }
+  template <int N, bool CFL>
+  void launch_passB64(int kxo, cpx<T>* tf, cpx<T>* pb, int nb) {
+    using B = PassB64<N>;
+    if constexpr (SplitB64<N>::OK) {
+      if (passb_mode_ == 2 && kxo == gd_.M) {  // three groups per row (small grids)
+        k_passB64_split<N, CFL><<<dim3(N, nb), SplitB64<N>::THREADS, SplitB64<N>::SMEM, st_>>>(
+            tf, pb, kxo, gd_, tw_, enc_base_, batch());
+        post("k_passB64_split");
+        return;
+      }
+    }
+    const int g = gb_ ? gb_ : Cfg<T, N>::G;  // groups per CTA: autotuned
+    const dim3 grid((N + g - 1) / g, nb);
+    if (kxo > gd_.M)
+      k_passB64<N, CFL, true><<<grid, B::TPF * g, g * B::GROUP, st_>>>(tf, pb, kxo, gd_, tw_, enc_base_, batch());
+    else
+      k_passB64<N, CFL, false><<<grid, B::TPF * g, g * B::GROUP, st_>>>(tf, pb, kxo, gd_, tw_, enc_base_, batch());
+    post("k_passB64");
+  }
+  // (FP64: the derivative planes are used up)
   template <bool CFL>
-  void launch_passB(int kxo, const cpx<T>* tf, cpx<T>* pb, int nb) {
+  void launch_passB(int kxo, cpx<T>* tf, cpx<T>* pb, int nb) {
+    if constexpr (sizeof(T) == 8)
+      dispatch_n(n_, [&](auto NC) { launch_passB64<decltype(NC)::value, CFL>(kxo, tf, pb, nb); });
+    else
+      launch_passB32<CFL>(kxo, tf, pb, nb);
+  }
+  template <bool CFL>
+  void launch_passB32(int kxo, cpx<T>* tf, cpx<T>* pb, int nb) {
     const T inv4 = (T)(1.0 / ((double)n_ * n_ * n_ * n_));
     dispatch_n(n_, [&](auto NC) {
       constexpr int N = decltype(NC)::value;
@@ -1142,7 +1200,14 @@ class EngineT final : public IEngine {
           post("k_passC_pipe");
         }
       }
-      if (!persistent) {  // one CTA (group) per column pair
+      if constexpr (sizeof(T) == 8) {  // one bracket of a column per CTA (group)
+        const int g = gc_ ? gc_ : C::G;  // groups per CTA: autotuned
+        const RkTab tab{rk_d1_, rk_d2_, rk_ik2_, rk_wk_, rk_run_};
+        k_passC64<N><<<dim3((gd_.M + g - 1) / g, nb, 2), C::TPF * g, g * kPassC64Group<N>, st_>>>(
+            pb_, c1in, c2in, pbase_[P_PS], pbase_[P_VZ], pbase_[P_FP], pbase_[P_FZ], c1out, c2out, gd_, tab,
+            scal_base_, o, tw_, batch(), t5, t6);
+        post("k_passC64");
+      } else if (!persistent) {  // one CTA (group) per column pair
         auto k = k_passC<T, N>;
         if constexpr (kFuseCA<T, N>) {
           if (fuse) k = k_passC<T, N, true>;
@@ -1172,7 +1237,7 @@ class EngineT final : public IEngine {
       constexpr size_t sm = Cfg<T, N>::SMEM;
       set_smem_attr(k_colfft<T, N, -1>, sm);
       set_smem_attr(k_colfft<T, N, +1>, sm);
-      set_smem_attr(k_colfft<T, N, -1, PassNT<T, N>::value>, sm);
+      set_smem_attr(k_colfft<T, N, -1, sizeof(T) == 8 ? 2 : PassNT<T, N>::value>, sm);
       set_smem_attr(k_rowc2r<T, N>, sm);
       set_smem_attr(k_rowr2c<T, N>, sm);
       set_smem_attr(k_cnn2_to_rows<T, N>, sm);
@@ -1180,15 +1245,40 @@ class EngineT final : public IEngine {
       set_smem_attr(k_colfft_band2<T, N>, sm);
       if constexpr (RowsCnn<T, N>::OK) set_smem_attr(k_rows_to_cnn8<T, N>, RowsCnn<T, N>::SMEM);
       constexpr size_t smh = PassSmem<T, N>::SMEM;
-      set_smem_attr(k_passA<T, N>, CfgA<T, N>::SMEM);
+      const auto carve = cudaFuncAttributePreferredSharedMemoryCarveout;
+      if constexpr (sizeof(T) == 8) {
+        // two CTAs per SM and more
+        cuda_check(cudaFuncSetAttribute(k_passA64<N>, carve, (int)cudaSharedmemCarveoutMaxShared), "carveout");
+        cuda_check(cudaFuncSetAttribute(k_passC64<N>, carve, (int)cudaSharedmemCarveoutMaxShared), "carveout");
+        set_smem_attr(k_passA64<N>, sm);
+        set_smem_attr(k_passC64<N>, Cfg<T, N>::G * kPassC64Group<N>);
+      } else {
+        set_smem_attr(k_passA<T, N>, CfgA<T, N>::SMEM);
+        set_smem_attr(k_passC<T, N>, smh);
+      }
       if constexpr (kAltRadixA<T, N>) set_smem_attr(k_passA<T, N, Cfg<T, N>::E>, CfgAE<T, N, Cfg<T, N>::E>::SMEM);
-      set_smem_attr(k_passB<T, N, true>, RolledB<T, N>::SMEM);
-      set_smem_attr(k_passB<T, N, false>, RolledB<T, N>::SMEM);
-      if constexpr (SplitB<T, N>::OK) {
+      if constexpr (sizeof(T) == 8) {
+        using B = PassB64<N>;
+        constexpr int G = Cfg<T, N>::G;
+        auto attr = [&](auto k, size_t smem) {
+          set_smem_attr(k, smem);
+          cuda_check(cudaFuncSetAttribute(k, carve, (int)cudaSharedmemCarveoutMaxShared), "carveout");
+        };
+        attr(k_passB64<N, true, false>, G * B::GROUP);
+        attr(k_passB64<N, false, false>, G * B::GROUP);
+        attr(k_passB64<N, false, true>, G * B::GROUP);
+        if constexpr (SplitB64<N>::OK) {
+          attr(k_passB64_split<N, true>, SplitB64<N>::SMEM);
+          attr(k_passB64_split<N, false>, SplitB64<N>::SMEM);
+        }
+      } else {
+        set_smem_attr(k_passB<T, N, true>, RolledB<T, N>::SMEM);
+        set_smem_attr(k_passB<T, N, false>, RolledB<T, N>::SMEM);
+      }
+      if constexpr (sizeof(T) == 4 && SplitB<T, N>::OK) {
         set_smem_attr(k_passB_split<T, N, true>, SplitB<T, N>::SMEM);
         set_smem_attr(k_passB_split<T, N, false>, SplitB<T, N>::SMEM);
       }
-      set_smem_attr(k_passC<T, N>, smh);
       if constexpr (kFuseCA<T, N>) set_smem_attr(k_passC<T, N, true>, smh);
       if constexpr (kPipeC<T, N>) {
         set_smem_attr(k_passC_pipe<N>, PipeC<N>::SMEM);
@@ -1331,7 +1421,7 @@ class EngineT final : public IEngine {
           cands.push_back({1, pipeb_ctas_});
           if (pipeb_ctas_ >= 2 * sms) cands.push_back({1, pipeb_ctas_ / 2});
         }
-        if constexpr (SplitB<T, N>::OK) cands.push_back({2, 1});
+        if constexpr (sizeof(T) == 8 ? SplitB64<N>::OK : SplitB<T, N>::OK) cands.push_back({2, 1});
         const std::vector<float> us = time_candidates(cands.size(), [&](size_t i) {
           passb_mode_ = cands[i].first;
           pipeb_grid_ = cands[i].first == 1 ? cands[i].second : 0;
@@ -1346,7 +1436,8 @@ class EngineT final : public IEngine {
       {
         cuda_check(cudaMemsetAsync(pb_, 0, sizeof(cpx<T>) * 2 * S_ * nb_, st_), "memset");
         cuda_check(cudaMemsetAsync(d_sc_, 0, sizeof(StepCoef) * nb_, st_), "memset");
-        coefs_valid_ = false;
+        build_rk_tables();
+        coefs_valid_ = sc_valid_ = false;
         struct CandC {
           int mode, grid, chunks, wide;
         };
@@ -1554,16 +1645,15 @@ class EngineT final : public IEngine {
 
  private:
   void build_twiddles() {
-    std::vector<double> c(n_), s(n_);
-    host_unit_roots(n_, c.data(), s.data());
     std::vector<tw_t<T>> h(n_), ha(n_);
     dispatch_n(n_, [&](auto NC) {
       constexpr int N = decltype(NC)::value;
       constexpr int EA = PassAE<T, N>::value;
       static_assert(BlockFFT<T, N, Cfg<T, N>::E>::TW_ELEMS <= N, "twiddle table fits in n entries");
       static_assert(BlockFFT<T, N, EA>::TW_ELEMS <= N, "twiddle table fits in n entries");
-      build_stage_twiddles<T, N, Cfg<T, N>::E>(h.data(), c.data(), s.data());
-      build_stage_twiddles<T, N, EA>(ha.data(), c.data(), s.data());
+      build_twiddle_table<T, N, Cfg<T, N>::E>(h.data());
+      if constexpr (EA == Cfg<T, N>::E) ha = h;
+      else build_twiddle_table<T, N, EA>(ha.data());
     });
     cuda_check(cudaMemcpyAsync(tw_, h.data(), sizeof(tw_t<T>) * n_, cudaMemcpyHostToDevice, st_), "H2D twiddles");
     cuda_check(cudaMemcpyAsync(tw_a_, ha.data(), sizeof(tw_t<T>) * n_, cudaMemcpyHostToDevice, st_),
@@ -1623,6 +1713,9 @@ class EngineT final : public IEngine {
   std::vector<ModelCoef> coefs_;
   std::vector<char> up_sc_, up_cc_;  // the coefficients on the device (upload_coefs)
   bool coefs_valid_ = false;
+  bool sc_valid_ = false;  // d_sc_ (and pass C's tables) hold up_sc_
+  double *rk_d1_ = nullptr, *rk_d2_ = nullptr, *rk_ik2_ = nullptr, *rk_wk_ = nullptr;  // FP64: RkTab
+  size_t rk_run_ = 0;
   cudaStream_t st_ = nullptr;
   bool ci_on_ = false;
   int ci_n_ = 0;

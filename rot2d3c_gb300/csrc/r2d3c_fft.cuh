@@ -1,4 +1,5 @@
-// Shared-memory / register block FFT for sm_103a.
+// Shared-memory / register block FFT for sm_103a: the FP32 transform and the
+// parts that the FP64 one (r2d3c_fx.cuh) shares.
 //
 // One length-N complex transform is carried by TPF = N/E threads.  Thread
 // `lane` holds v[q] = x[lane + q*TPF] (q < E) on entry and X[lane + q*TPF] on
@@ -10,8 +11,8 @@
 // a smaller radix), each an in-register DFT of R points followed by one padded
 // shared-memory exchange.  NT transforms can be carried at once by the same
 // threads; they share the twiddle loads and the barriers.  Twiddles come from a per-N table
-// tw[k] = exp(-2*pi*i*k/N) built on the host in FP64; the FP32 path stores
-// every twiddle as an (hi, lo) float pair and applies the low part with an
+// tw[k] = exp(-2*pi*i*k/N) built on the host in FP64; they are stored
+// as (hi, lo) float pairs and applied with the low part in an
 // extra FMA ("compensated twiddles"), which removes the twiddle rounding from
 // the FP32 error budget.
 #pragma once
@@ -28,9 +29,10 @@ template <> struct V2<double> { using t = double2; };
 template <> struct V2<float> { using t = float2; };
 template <typename T> using cpx = typename V2<T>::t;
 
-// Twiddle storage: FP64 -> (re, im); FP32 -> (re_hi, im_hi, re_lo, im_lo).
+// Twiddle storage: FP64 -> fixed-point limbs (r2d3c_fx.cuh); FP32 -> (re_hi,
+// im_hi, re_lo, im_lo).
 template <typename T> struct TwS;
-template <> struct TwS<double> { using t = double2; };
+template <> struct TwS<double> { using t = int4; };
 template <> struct TwS<float> { using t = float4; };
 template <typename T> using tw_t = typename TwS<T>::t;
 
@@ -46,11 +48,6 @@ __device__ __forceinline__ cpx<T> mkc(T x, T y) {
 
 // a * w with w from the table; DIR = -1 uses w, DIR = +1 uses conj(w).
 template <int DIR>
-__device__ __forceinline__ double2 twmul(double2 a, double2 w) {
-  const double wy = DIR < 0 ? w.y : -w.y;
-  return make_double2(fma(a.x, w.x, -a.y * wy), fma(a.x, wy, a.y * w.x));
-}
-template <int DIR>
 __device__ __forceinline__ float2 twmul(float2 a, float4 w) {
   const float wy = DIR < 0 ? w.y : -w.y;
   const float ly = DIR < 0 ? w.w : -w.w;
@@ -61,7 +58,7 @@ __device__ __forceinline__ float2 twmul(float2 a, float4 w) {
 }
 
 // Constant twiddle exp(DIR*2*pi*i*I16/16), I16 in [0,8).  The constants are
-// cos/sin of multiples of pi/8; the FP32 variant carries a low-order part.
+// cos/sin of multiples of pi/8 with a low-order part.
 template <typename T, int I16, int DIR>
 __device__ __forceinline__ cpx<T> kmul(cpx<T> a) {
   constexpr double C1 = 0.92387953251128675613;  // cos(pi/8)
@@ -84,15 +81,11 @@ __device__ __forceinline__ cpx<T> kmul(cpx<T> a) {
     constexpr double c = (I16 == 1) ? C1 : (I16 == 3) ? S1 : (I16 == 5) ? -S1 : -C1;
     constexpr double s = (I16 == 1) ? S1 : (I16 == 3) ? C1 : (I16 == 5) ? C1 : S1;
     constexpr double sd = DIR * s;
-    if constexpr (sizeof(T) == 8) {
-      return mkc<T>(fma(a.x, c, -a.y * sd), fma(a.x, sd, a.y * c));
-    } else {
-      constexpr float ch = (float)c, cl = (float)(c - (double)(float)c);
-      constexpr float sh = (float)sd, sl = (float)(sd - (double)(float)sd);
-      const float tr = fmaf(a.x, cl, -a.y * sl);
-      const float ti = fmaf(a.x, sl, a.y * cl);
-      return mkc<T>(fmaf(a.x, ch, fmaf(-a.y, sh, tr)), fmaf(a.x, sh, fmaf(a.y, ch, ti)));
-    }
+    constexpr float ch = (float)c, cl = (float)(c - (double)(float)c);
+    constexpr float sh = (float)sd, sl = (float)(sd - (double)(float)sd);
+    const float tr = fmaf(a.x, cl, -a.y * sl);
+    const float ti = fmaf(a.x, sl, a.y * cl);
+    return mkc<T>(fmaf(a.x, ch, fmaf(-a.y, sh, tr)), fmaf(a.x, sh, fmaf(a.y, ch, ti)));
   }
 }
 
@@ -308,10 +301,6 @@ inline void host_unit_roots(int n, double* c, double* s) {
   }
 }
 
-inline void fill_tw(double2& w, double re, double im) {
-  w.x = re;
-  w.y = im;
-}
 inline void fill_tw(float4& w, double re, double im) {
   w.x = (float)re;
   w.y = (float)im;

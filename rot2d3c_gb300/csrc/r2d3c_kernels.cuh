@@ -7,7 +7,8 @@
 //   mixed plane     T[kx][y]   result of the y-direction transform of one kx
 //                   column, y fastest; used between the column and row passes
 //
-// Hot path of one RK substep (Rot2D3C.para.f90:571-599), three passes:
+// Hot path of one RK substep (Rot2D3C.para.f90:571-599), three passes (the
+// FP32 kernels here, the FP64 ones in r2d3c_pass64.cuh):
 //   A  per kx column (kx <= n/3): the six masked spectral derivatives
 //      d_x psi, d_y psi, d_x(-k^2 psi), d_y(-k^2 psi), d_x vz, d_y vz
 //      (derivk2/laplak2, pseudospec2D_Rot2D3C.f90:6-95) and their inverse
@@ -24,7 +25,7 @@
 
 #include <type_traits>
 
-#include "r2d3c_fft.cuh"
+#include "r2d3c_fx.cuh"
 
 namespace r2d3c {
 
@@ -66,8 +67,8 @@ struct Cfg {
 // FP32 path up to n = 4096 ("tiled" mode): pass A and C transform two
 // adjacent kx columns, pass B two adjacent rows, and the mixed planes use the
 // pair-tiled layout below so that every access moves whole 32-byte sectors.
-// One in the FP64 path (its FP64 arithmetic is the bound and its register
-// budget is full) and at n = 8192: plain column layout T[kx][y].
+// One at n = 8192 (plain column layout T[kx][y]) and in the FP64 path, which
+// has passes of its own (r2d3c_pass64.cuh).
 template <typename T, int N> struct PassNT {
   static constexpr int value = (sizeof(T) == 4 && N <= 4096) ? 2 : 1;
 };
@@ -90,8 +91,8 @@ using CfgAE = Cfg<T, N, PassNT<T, N>::value, EA, EA != 16>;
 template <typename T, int N>
 constexpr bool kAltRadixA = PassAE<T, N>::value != Cfg<T, N>::E;
 
-// Shared memory of passes B and C: NT transform buffers per group, plus (when
-// it fits) a store for the first transform's result, which is held across the
+// Shared memory of passes B and C: NT transform buffers per group, plus a
+// store for the first transform's result, which is held across the
 // later transforms (pass B: dx psi + i dy psi; pass C: the [psi,-k^2 psi]
 // column) -- keeping it out of registers avoids spills.
 template <typename T, int N>
@@ -99,8 +100,8 @@ struct PassSmem {
   static constexpr int NT = PassNT<T, N>::value;
   using C = Cfg<T, N, NT>;
   static constexpr size_t HOLD_BYTES = (size_t)NT * N * sizeof(cpx<T>);
-  static constexpr bool HOLD = C::FFT::SMEM_BYTES + HOLD_BYTES <= 200 * 1024;
-  static constexpr size_t GROUP_ELEMS = (size_t)NT * C::FFT::SMEM_ELEMS + (HOLD ? (size_t)NT * N : 0);
+  static_assert(sizeof(T) == 8 || C::FFT::SMEM_BYTES + HOLD_BYTES <= 200 * 1024, "fits an SM");
+  static constexpr size_t GROUP_ELEMS = (size_t)NT * C::FFT::SMEM_ELEMS + (size_t)NT * N;
   static constexpr size_t SMEM = (size_t)C::G * GROUP_ELEMS * sizeof(cpx<T>);
 };
 
@@ -460,7 +461,7 @@ __device__ __forceinline__ void cfl_max_sq(const cpx<T> (&v)[NT][E], unsigned lo
 // of the conjugate, conjugated: bit-identical to the unrolled form.
 template <typename T, int N>
 struct RolledB {
-  static constexpr bool OK = sizeof(T) == 4 && PassNT<T, N>::value == 1 && PassSmem<T, N>::HOLD;
+  static constexpr bool OK = sizeof(T) == 4 && PassNT<T, N>::value == 1;
   static constexpr size_t SMEM = PassSmem<T, N>::SMEM + (OK ? (size_t)Cfg<T, N, 1>::G * N * sizeof(T) : 0);
 };
 
@@ -470,7 +471,6 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
         const tw_t<T>* __restrict__ tw, unsigned long long* __restrict__ cfl_enc, Batch bs) {
   constexpr int NR = PassNT<T, N>::value;
   using PS = PassSmem<T, N>;
-  constexpr bool HOLD = PS::HOLD;
   tf += blockIdx.y * bs.tf;
   pb += blockIdx.y * bs.pb;
   cfl_enc += blockIdx.y * kScalStride;
@@ -479,7 +479,7 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
   R2D3C_SMEM_DECL
   const int g = threadIdx.x / C::TPF, lane = threadIdx.x % C::TPF;
   cpx<T>* sm = smbase_ + (size_t)g * PS::GROUP_ELEMS;
-  cpx<T>* hold = sm + NR * F::SMEM_ELEMS;  // z1 store (HOLD)
+  cpx<T>* hold = sm + NR * F::SMEM_ELEMS;  // z1 store
   int rg = blockIdx.x * (blockDim.x / C::TPF) + g;  // groups per CTA: a launch-time choice
   const bool ok = rg < N / NR;
   if (!ok) rg = 0;  // surplus groups recompute rows 0.. and store nothing
@@ -527,7 +527,6 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
       }
     }
   } else {
-  cpx<T> z1r[HOLD ? 1 : NR][C::E];
   T p1[NR][C::E];
   // pair (d_x psi, d_y psi)
 #pragma unroll
@@ -540,17 +539,11 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
   F::template run<+1>(v, lane, sm, tw);
   if constexpr (CFL) cfl_max_sq<T, NR, C::E>(v, cfl_enc);
   // each thread reads back only the positions it wrote: no barrier needed
-  auto z1 = [&](int t, int q) -> cpx<T> {
-    if constexpr (HOLD) return hold[t * N + lane + q * C::TPF];
-    else return z1r[t][q];
-  };
+  auto z1 = [&](int t, int q) -> cpx<T> { return hold[t * N + lane + q * C::TPF]; };
 #pragma unroll
   for (int t = 0; t < NR; ++t)
 #pragma unroll
-    for (int q = 0; q < C::E; ++q) {
-      if constexpr (HOLD) hold[t * N + lane + q * C::TPF] = v[t][q];
-      else z1r[t][q] = v[t][q];
-    }
+    for (int q = 0; q < C::E; ++q) hold[t * N + lane + q * C::TPF] = v[t][q];
   // pair (d_x(-k^2 psi), d_y(-k^2 psi)) -> [psi, -k^2 psi]
 #pragma unroll
   for (int q = 0; q < C::E; ++q) {
@@ -944,18 +937,6 @@ struct RkIn {
   cpx<T> a1, a2, p0, f0, v0, g0;
 };
 
-template <typename T>
-__device__ __forceinline__ void rk_load(RkIn<T>& r, size_t idx, const cpx<T>* c1in, const cpx<T>* c2in,
-                                        const cpx<T>* ps, const cpx<T>* vz, const cpx<T>* __restrict__ fp,
-                                        const cpx<T>* __restrict__ fz) {
-  r.a1 = c1in[idx];
-  r.a2 = c2in[idx];
-  r.p0 = ps[idx];
-  r.f0 = fp[idx];
-  r.v0 = vz[idx];
-  r.g0 = fz[idx];
-}
-
 // New C1 (rk_apply1) and C2 (rk_apply2) of one element
 // (Rot2D3C.para.f90:580-599); zero outside the retained disc and at k = 0.
 // Both components are divided by the same implicit divisor: one reciprocal
@@ -989,13 +970,6 @@ __device__ __forceinline__ cpx<T> rk_apply2(const RkIn<T>& r, const cpx<T> c6, i
   const T r3v = (T)1 / tmp3v;
   return mkc<T>(u2x * r3v, u2y * r3v);
 }
-template <typename T>
-__device__ __forceinline__ void rk_apply(const RkIn<T>& r, const cpx<T> c5, const cpx<T> c6, int kyi, int k2,
-                                         const StepCoef& sc, T tmp1, cpx<T>& n1, cpx<T>& n2) {
-  n1 = rk_apply1<T>(r, c5, kyi, k2, sc, tmp1);
-  n2 = rk_apply2<T>(r, c6, kyi, k2, sc, tmp1);
-}
-
 // L2 prefetch (cp.async.bulk.prefetch, no completion to wait for) of the
 // retained rows |ky| <= L of ncol adjacent spectral columns starting at p:
 // rows [0, L] of the first column, then each run [N - L, N + L] across a
@@ -1155,7 +1129,6 @@ k_passC(const cpx<T>* __restrict__ pb, const cpx<T>* c1in, const cpx<T>* c2in,
         const tw_t<T>* __restrict__ twa = nullptr) {
   constexpr int NT = PassNT<T, N>::value;
   using PS = PassSmem<T, N>;
-  constexpr bool HOLD = PS::HOLD;
   const size_t rs = blockIdx.y * bs.spec;
   pb += blockIdx.y * bs.pb;
   c1in += rs;
@@ -1171,11 +1144,11 @@ k_passC(const cpx<T>* __restrict__ pb, const cpx<T>* c1in, const cpx<T>* c2in,
   R2D3C_SMEM_DECL
   const int g = threadIdx.x / C::TPF, lane0 = threadIdx.x % C::TPF;
   cpx<T>* sm = smbase_ + (size_t)g * PS::GROUP_ELEMS;
-  cpx<T>* hold = sm + NT * F::SMEM_ELEMS;  // transformed [psi,-k^2 psi] columns (HOLD)
-  // wide > 1 (FP32 grids with the held c5): a team of `wide` groups per
+  cpx<T>* hold = sm + NT * F::SMEM_ELEMS;  // transformed [psi,-k^2 psi] columns
+  // wide > 1: a team of `wide` groups per
   // column pair; each group transforms (the same values), and the team
   // shares the RK update, which is the longer part of small grids' chain
-  const int W = (HOLD && sizeof(T) == 4) ? wide : 1;
+  const int W = wide;
   const int team = g / W, member = g % W;
   const int kx0 = (blockIdx.x * ((blockDim.x / C::TPF) / W) + team) * NT;  // groups per CTA: a launch-time choice
   const size_t oplane = (size_t)gd.nh * N;
@@ -1189,17 +1162,15 @@ k_passC(const cpx<T>* __restrict__ pb, const cpx<T>* c1in, const cpx<T>* c2in,
     // with two chunks each CTA needs half of them: z = 0 the C1 update's
     // (c2in, ps, fp, tau5), z = 1 the C2 update's (c1in, vz, fz, tau6)
     const int user = lane < 2 ? 1 - lane : (lane & 1);  // the chunk that reads src
-    const bool need = gridDim.z == 1 || !(sizeof(T) == 4 && HOLD) || (int)blockIdx.z == user;
+    const bool need = gridDim.z == 1 || (int)blockIdx.z == user;
     const int ncol = min(NT, gd.M - kx0);
     if (src && need && ncol > 0) prefetch_columns_l2<T>(src + (size_t)kx0 * N, ncol, N, gd.L);
   }
   cpx<T> v[NT][C::E];
-  cpx<T> c5r[HOLD ? 1 : NT][C::E];
-  // gridDim.z = 2 splits a column pair's work over two CTAs (FP32 grids with
-  // the held c5): z = 0 transforms [psi,-k^2 psi] and updates C1, z = 1
+  // gridDim.z = 2 splits a column pair's work over two CTAs: z = 0 transforms [psi,-k^2 psi] and updates C1, z = 1
   // transforms [psi, vz] and updates C2; the arithmetic per element is the
   // same as with one CTA (the launch autotuner chooses)
-  const int chunk = (HOLD && sizeof(T) == 4 && gridDim.z > 1) ? (int)blockIdx.z : -1;
+  const int chunk = gridDim.z > 1 ? (int)blockIdx.z : -1;
 #pragma unroll 1
   for (int pl = 0; pl < 2; ++pl) {
     if (chunk >= 0 && pl != chunk) continue;
@@ -1240,8 +1211,7 @@ k_passC(const cpx<T>* __restrict__ pb, const cpx<T>* c1in, const cpx<T>* c2in,
       for (int t = 0; t < NT; ++t)
 #pragma unroll
         for (int q = 0; q < C::E; ++q) {
-          if constexpr (HOLD) hold[t * N + lane + q * C::TPF] = v[t][q];
-          else c5r[t][q] = v[t][q];
+          hold[t * N + lane + q * C::TPF] = v[t][q];
         }
     }
   }
@@ -1250,145 +1220,67 @@ k_passC(const cpx<T>* __restrict__ pb, const cpx<T>* c1in, const cpx<T>* c2in,
   // read only now, not held in registers across the transforms.
   const StepCoef sc = scs[blockIdx.y];
   const T tmp1 = (T)(scal[blockIdx.y * kScalStride] / (double)o);  // :581
-  if constexpr (HOLD && sizeof(T) == 4) {
-    cpx<T>* lsm = smbase_ + (size_t)(team * W) * PS::GROUP_ELEMS;  // the team's first group
-    passC_update_pairs<T, N, NT, C::E, C::TPF>(lsm, lsm + NT * F::SMEM_ELEMS, v, lane, kx0, c1in, c2in, ps, vz, fp,
-                                                fz, c1out, c2out, gd, sc, tmp1, tau5, tau6, chunk, member * C::TPF + lane,
-                                                W * C::TPF, member == 0);
-    if constexpr (ATAIL) {
-      using CA = CfgA<T, N>;
-      static_assert(NT == 2 && std::is_same<typename CA::FFT, F>::value && CA::TPF == C::TPF,
-                    "pass A's transform configuration is pass C's");
-      // the team's update stores (and its reads of the shared staging) are
-      // done: the state written is visible to the whole CTA
-      __syncthreads();
-      // fields 0-3 from the new psi (C1), 4-5 from the new vz (C2); a CTA of
-      // a chunked launch takes its own update's fields.  Every group runs the
-      // same number of transforms (their barriers are CTA-wide above 32
-      // threads per transform); a group without a field transforms zeros and
-      // stores nothing.
-      const int fb = chunk == 1 ? 4 : 0, fe = chunk == 0 ? 4 : 6;
-      const int rounds = (fe - fb + W - 1) / W;
-      const size_t plane = (size_t)gd.M * N;
-      cpx<T>* tsm = smbase_ + (size_t)g * PS::GROUP_ELEMS;  // this group's transform buffers
+  cpx<T>* lsm = smbase_ + (size_t)(team * W) * PS::GROUP_ELEMS;  // the team's first group
+  passC_update_pairs<T, N, NT, C::E, C::TPF>(lsm, lsm + NT * F::SMEM_ELEMS, v, lane, kx0, c1in, c2in, ps, vz, fp,
+                                              fz, c1out, c2out, gd, sc, tmp1, tau5, tau6, chunk, member * C::TPF + lane,
+                                              W * C::TPF, member == 0);
+  if constexpr (ATAIL) {
+    using CA = CfgA<T, N>;
+    static_assert(NT == 2 && std::is_same<typename CA::FFT, F>::value && CA::TPF == C::TPF,
+                  "pass A's transform configuration is pass C's");
+    // the team's update stores (and its reads of the shared staging) are
+    // done: the state written is visible to the whole CTA
+    __syncthreads();
+    // fields 0-3 from the new psi (C1), 4-5 from the new vz (C2); a CTA of
+    // a chunked launch takes its own update's fields.  Every group runs the
+    // same number of transforms (their barriers are CTA-wide above 32
+    // threads per transform); a group without a field transforms zeros and
+    // stores nothing.
+    const int fb = chunk == 1 ? 4 : 0, fe = chunk == 0 ? 4 : 6;
+    const int rounds = (fe - fb + W - 1) / W;
+    const size_t plane = (size_t)gd.M * N;
+    cpx<T>* tsm = smbase_ + (size_t)g * PS::GROUP_ELEMS;  // this group's transform buffers
 #pragma unroll 1
-      for (int r = 0; r < rounds; ++r) {
-        const int f = fb + member + r * W;
-        const bool act = f < fe;
-        const cpx<T>* sp = f < 4 ? c1out : c2out;
-        cpx<T> a[NT][C::E];
+    for (int r = 0; r < rounds; ++r) {
+      const int f = fb + member + r * W;
+      const bool act = f < fe;
+      const cpx<T>* sp = f < 4 ? c1out : c2out;
+      cpx<T> a[NT][C::E];
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          const int col = kx0 + t;
-#pragma unroll
-          for (int q = 0; q < C::E; ++q) {
-            const int ky = ky_of(lane + q * C::TPF, N);
-            const bool in = act && col < gd.M && (ky <= gd.L && -ky <= gd.L) && col * col + ky * ky <= gd.kmaxi;
-            cpx<T> x = in ? sp[(size_t)col * N + lane + q * C::TPF] : czero<T>();
-            // (0,k)*(x,y) = (-k*y, k*x): derivk2 dir 1 (k = kx) / dir 2 (k = ky)
-            const T k = (f & 1) ? (T)ky : (T)col;
-            if (f == 2 || f == 3) {
-              const T m = -(T)(col * col + ky * ky);  // laplak2: -ka2*a
-              x = mkc<T>(m * x.x, m * x.y);
-            }
-            a[t][q] = mkc<T>(-k * x.y, k * x.x);
-          }
-        }
-        F::template run<+1>(a, lane, tsm, twa);
-        // lanes (2p, 2p+1) hold rows y = 2p, 2p+1 of columns kx0, kx0+1: one
-        // swap, then each lane writes one column's row pair (16 bytes)
-        const bool odd = lane & 1;
-        const int kx = kx0 + (odd ? 1 : 0);
-        cpx<T>* dst = atf + (size_t)(act ? f : 0) * plane;
+      for (int t = 0; t < NT; ++t) {
+        const int col = kx0 + t;
 #pragma unroll
         for (int q = 0; q < C::E; ++q) {
-          const cpx<T> give = odd ? a[0][q] : a[1][q];
-          cpx<T> got;
-          got.x = __shfl_xor_sync(0xffffffffu, give.x, 1);
-          got.y = __shfl_xor_sync(0xffffffffu, give.y, 1);
-          const int y = (lane + q * C::TPF) & ~1;
-          if (act && kx < gd.M) {
-            const cpx<T> lo = odd ? got : a[0][q];
-            const cpx<T> hi = odd ? a[1][q] : got;
-            *reinterpret_cast<float4*>(dst + mix_idx<N, 2>(kx, y, gd.M)) = make_float4(lo.x, lo.y, hi.x, hi.y);
+          const int ky = ky_of(lane + q * C::TPF, N);
+          const bool in = act && col < gd.M && (ky <= gd.L && -ky <= gd.L) && col * col + ky * ky <= gd.kmaxi;
+          cpx<T> x = in ? sp[(size_t)col * N + lane + q * C::TPF] : czero<T>();
+          // (0,k)*(x,y) = (-k*y, k*x): derivk2 dir 1 (k = kx) / dir 2 (k = ky)
+          const T k = (f & 1) ? (T)ky : (T)col;
+          if (f == 2 || f == 3) {
+            const T m = -(T)(col * col + ky * ky);  // laplak2: -ka2*a
+            x = mkc<T>(m * x.x, m * x.y);
           }
+          a[t][q] = mkc<T>(-k * x.y, k * x.x);
         }
       }
-    }
-  } else if constexpr (HOLD) {
-    // c6 joins c5 in shared memory (the transform buffer is free after the
-    // last transform; each thread reads back only what it wrote), and the
-    // update runs over this thread's elements in batches of RB: all loads of
-    // a batch, then its arithmetic and stores.
-    cpx<T>* c6s = sm;
-#pragma unroll
-    for (int t = 0; t < NT; ++t)
-#pragma unroll
-      for (int q = 0; q < C::E; ++q) c6s[t * N + lane + q * C::TPF] = v[t][q];
-    constexpr int NE = NT * C::E, RB = 2;
-    static_assert(NE % RB == 0, "whole batches");
-#pragma unroll 1
-    for (int e0 = 0; e0 < NE; e0 += RB) {
-      RkIn<T> in[RB];
-      cpx<T> ta[RB], tb[RB];
-#pragma unroll
-      for (int b = 0; b < RB; ++b) {
-        const int t = (e0 + b) / C::E, q = (e0 + b) % C::E;
-        const int col = kx0 + t, j = lane + q * C::TPF, ky = ky_of(j, N), k2 = col * col + ky * ky;
-        if (col < gd.M && k2 <= gd.kmaxi && k2 >= 1) {
-          const size_t idx = (size_t)col * N + j;
-          rk_load<T>(in[b], idx, c1in, c2in, ps, vz, fp, fz);
-          if (tau5) {
-            ta[b] = tau5[idx];
-            tb[b] = tau6[idx];
-          }
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < RB; ++b) {
-        const int t = (e0 + b) / C::E, q = (e0 + b) % C::E;
-        const int col = kx0 + t, j = lane + q * C::TPF, ky = ky_of(j, N), k2 = col * col + ky * ky;
-        if (col >= gd.M || ky > gd.L || -ky > gd.L) continue;
-        cpx<T> n1 = czero<T>(), n2 = czero<T>();
-        if (k2 <= gd.kmaxi && k2 >= 1) {  // ka2 <= kmax .and. ka2 > tiny (:580)
-          cpx<T> c5 = hold[t * N + j], c6 = c6s[t * N + j];
-          if (tau5) {  // learned subgrid tendencies of the two brackets
-            c5 = mkc<T>(c5.x + ta[b].x, c5.y + ta[b].y);
-            c6 = mkc<T>(c6.x + tb[b].x, c6.y + tb[b].y);
-          }
-          rk_apply<T>(in[b], c5, c6, ky, k2, sc, tmp1, n1, n2);
-        }
-        const size_t idx = (size_t)col * N + j;
-        c1out[idx] = n1;
-        c2out[idx] = n2;
-      }
-    }
-  } else {
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      const int col = kx0 + t;
-      if (col >= gd.M) continue;
+      F::template run<+1>(a, lane, tsm, twa);
+      // lanes (2p, 2p+1) hold rows y = 2p, 2p+1 of columns kx0, kx0+1: one
+      // swap, then each lane writes one column's row pair (16 bytes)
+      const bool odd = lane & 1;
+      const int kx = kx0 + (odd ? 1 : 0);
+      cpx<T>* dst = atf + (size_t)(act ? f : 0) * plane;
 #pragma unroll
       for (int q = 0; q < C::E; ++q) {
-        const int j = lane + q * C::TPF;
-        const int ky = ky_of(j, N);
-        if (ky > gd.L || -ky > gd.L) continue;
-        const int k2 = col * col + ky * ky;
-        cpx<T> n1 = czero<T>(), n2 = czero<T>();
-        const size_t idx = (size_t)col * N + j;
-        if (k2 <= gd.kmaxi && k2 >= 1) {
-          cpx<T> c5 = c5r[t][q], c6 = v[t][q];
-          if (tau5) {
-            const cpx<T> a = tau5[idx], b = tau6[idx];
-            c5 = mkc<T>(c5.x + a.x, c5.y + a.y);
-            c6 = mkc<T>(c6.x + b.x, c6.y + b.y);
-          }
-          RkIn<T> in;
-          rk_load<T>(in, idx, c1in, c2in, ps, vz, fp, fz);
-          rk_apply<T>(in, c5, c6, ky, k2, sc, tmp1, n1, n2);
+        const cpx<T> give = odd ? a[0][q] : a[1][q];
+        cpx<T> got;
+        got.x = __shfl_xor_sync(0xffffffffu, give.x, 1);
+        got.y = __shfl_xor_sync(0xffffffffu, give.y, 1);
+        const int y = (lane + q * C::TPF) & ~1;
+        if (act && kx < gd.M) {
+          const cpx<T> lo = odd ? got : a[0][q];
+          const cpx<T> hi = odd ? a[1][q] : got;
+          *reinterpret_cast<float4*>(dst + mix_idx<N, 2>(kx, y, gd.M)) = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
-        c1out[idx] = n1;
-        c2out[idx] = n2;
       }
     }
   }
@@ -1416,14 +1308,14 @@ struct PipeC {
 // pass C may split a column pair's C1 and C2 updates over two CTAs (gridDim.z
 // = 2) where it holds c5 in shared memory and updates row pairs (FP32)
 template <typename T, int N>
-constexpr bool kChunkC = sizeof(T) == 4 && PassSmem<T, N>::HOLD;
+constexpr bool kChunkC = sizeof(T) == 4;
 // pass C carries the next substep's pass A (k_passC<T, N, true>): FP32 grids
 // whose pass A and pass C share one transform configuration
 template <typename T, int N>
-constexpr bool kFuseCA = sizeof(T) == 4 && N <= 512 && PassNT<T, N>::value == 2 && PassSmem<T, N>::HOLD &&
+constexpr bool kFuseCA = sizeof(T) == 4 && N <= 512 && PassNT<T, N>::value == 2 &&
                          !kAltRadixA<T, N> && PassAE<T, N>::value == Cfg<T, N>::E;
 template <typename T, int N>
-constexpr bool kPipeC = sizeof(T) == 4 && PassNT<T, N>::value == 2 && PassSmem<T, N>::HOLD &&
+constexpr bool kPipeC = sizeof(T) == 4 && PassNT<T, N>::value == 2 &&
                         PipeC<N>::THREADS >= 64 && PipeC<N>::THREADS <= 512;
 
 template <int N>

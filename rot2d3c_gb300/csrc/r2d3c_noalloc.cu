@@ -50,12 +50,12 @@ constexpr int kTwElems = 2 * kNoAllocMaxN - 16;
 constexpr int kMaxDevices = 64;
 
 static __device__ __align__(256) double2 g_noalloc_scratch[kScratchElems];
-static __device__ __align__(256) double2 g_noalloc_tw[kTwElems];
+static __device__ __align__(256) int4 g_noalloc_tw[kTwElems];
 
 struct DevSlot {
   std::atomic<bool> ready{false};  // published (release) once the fields below are set
   double2* scratch = nullptr;  // device address of g_noalloc_scratch
-  double2* tw = nullptr;       // device address of g_noalloc_tw
+  int4* tw = nullptr;          // device address of g_noalloc_tw
 };
 DevSlot g_slots[kMaxDevices];
 std::mutex g_mu;
@@ -66,18 +66,16 @@ int tw_offset(int n) {  // start of the n-point table inside g_noalloc_tw
   return off;
 }
 
-// The stage-major tables of the column and row kernels for one n, from the
-// same FP64 roots as the engines' tables.
-void host_twiddles(int n, double2* out) {
-  std::vector<double> c(n), s(n);
-  host_unit_roots(n, c.data(), s.data());
+// The stage-major tables of the column and row kernels for one n, as the
+// engines'.
+void host_twiddles(int n, int4* out) {
   switch (n) {
-    case 16: build_stage_twiddles<double, 16, Cfg<double, 16>::E>(out, c.data(), s.data()); break;
-    case 32: build_stage_twiddles<double, 32, Cfg<double, 32>::E>(out, c.data(), s.data()); break;
-    case 64: build_stage_twiddles<double, 64, Cfg<double, 64>::E>(out, c.data(), s.data()); break;
-    case 128: build_stage_twiddles<double, 128, Cfg<double, 128>::E>(out, c.data(), s.data()); break;
-    case 256: build_stage_twiddles<double, 256, Cfg<double, 256>::E>(out, c.data(), s.data()); break;
-    default: build_stage_twiddles<double, 512, Cfg<double, 512>::E>(out, c.data(), s.data()); break;
+    case 16: build_twiddle_table<double, 16, Cfg<double, 16>::E>(out); break;
+    case 32: build_twiddle_table<double, 32, Cfg<double, 32>::E>(out); break;
+    case 64: build_twiddle_table<double, 64, Cfg<double, 64>::E>(out); break;
+    case 128: build_twiddle_table<double, 128, Cfg<double, 128>::E>(out); break;
+    case 256: build_twiddle_table<double, 256, Cfg<double, 256>::E>(out); break;
+    default: build_twiddle_table<double, 512, Cfg<double, 512>::E>(out); break;
   }
 }
 
@@ -89,9 +87,9 @@ DevSlot& setup(int dev) {
   if (s.ready.load(std::memory_order_acquire)) return s;  // set-up done: no lock on the call path
   std::lock_guard<std::mutex> lk(g_mu);
   if (s.ready.load(std::memory_order_relaxed)) return s;
-  std::vector<double2> h(kTwElems);
+  std::vector<int4> h(kTwElems);
   for (int n = 16; n <= kNoAllocMaxN; n <<= 1) host_twiddles(n, h.data() + tw_offset(n));
-  cuda_check(cudaMemcpyToSymbol(g_noalloc_tw, h.data(), sizeof(double2) * kTwElems),
+  cuda_check(cudaMemcpyToSymbol(g_noalloc_tw, h.data(), sizeof(int4) * kTwElems),
              "cudaMemcpyToSymbol(no-alloc twiddles)");
   // A copy from pageable host memory may return before its DMA has landed,
   // and the kernels run on the caller's stream, which need not wait for the
@@ -102,14 +100,14 @@ DevSlot& setup(int dev) {
   s.scratch = static_cast<double2*>(p);
   p = nullptr;
   cuda_check(cudaGetSymbolAddress(&p, g_noalloc_tw), "cudaGetSymbolAddress(no-alloc twiddles)");
-  s.tw = static_cast<double2*>(p);
+  s.tw = static_cast<int4*>(p);
   // the column and row kernels of every n use dynamic shared memory below 48 KB
   s.ready.store(true, std::memory_order_release);
   return s;
 }
 
 template <int N>
-void launch(const double2* in, double* out, double2* scratch, const double2* tw, cudaStream_t st) {
+void launch(const double2* in, double* out, double2* scratch, const int4* tw, cudaStream_t st) {
   using C = Cfg<double, N, 1>;
   static_assert(C::SMEM <= 48 * 1024, "no-alloc sizes stay below the default shared-memory limit");
   k_colfft<double, N, +1><<<(N / 2 + 1 + C::G - 1) / C::G, C::THREADS, C::SMEM, st>>>(in, scratch, N / 2 + 1,
@@ -133,7 +131,7 @@ extern "C" int r2d3c_fft_c2r_noalloc(int n, const double* d_in, double* d_out, v
     if (dev < 0 || dev >= kMaxDevices) throw Error(kEINVAL, "device index out of range");
     DevSlot& s = setup(dev);
     const double2* in = reinterpret_cast<const double2*>(d_in);
-    const double2* tw = s.tw + tw_offset(n);
+    const int4* tw = s.tw + tw_offset(n);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch (n) {
       case 16: launch<16>(in, d_out, s.scratch, tw, st); break;
