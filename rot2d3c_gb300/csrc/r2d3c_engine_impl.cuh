@@ -14,6 +14,7 @@
 
 #include "r2d3c_aux.cuh"
 #include "r2d3c_engine.h"
+#include "r2d3c_pass32.cuh"
 #include "r2d3c_pass64.cuh"
 
 namespace r2d3c {
@@ -33,6 +34,17 @@ void dispatch_n(int n, F&& f) {
     case 8192: f(std::integral_constant<int, 8192>{}); break;
     default: throw Error(kEINVAL, "unsupported grid size n");
   }
+}
+
+// The split of an SM's 256 KB between shared memory and L1 that just holds
+// `ctas` CTAs of `smem` bytes (and the 1 KB each that the system takes): the
+// transforms' twiddle tables (64 KB at n = 4096) live in what is left as L1.
+template <typename K>
+inline void set_carveout(K kernel, size_t smem, int ctas) {
+  const size_t need = (smem + 1024) * (size_t)ctas, all = 228 * 1024;
+  const int pct = (int)std::min<size_t>(100, (need * 100 + all - 1) / all);
+  cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct),
+             "cudaFuncSetAttribute(carveout)");
 }
 
 template <typename K>
@@ -1130,7 +1142,7 @@ class EngineT final : public IEngine {
       k_passB64<N, CFL, false><<<grid, B::TPF * g, g * B::GROUP, st_>>>(tf, pb, kxo, gd_, tw_, enc_base_, batch());
     post("k_passB64");
   }
-  // (FP64: the derivative planes are used up)
+  // (FP64, and FP32 from n = 2048: the derivative planes are used up)
   template <bool CFL>
   void launch_passB(int kxo, cpx<T>* tf, cpx<T>* pb, int nb) {
     if constexpr (sizeof(T) == 8)
@@ -1145,36 +1157,49 @@ class EngineT final : public IEngine {
       constexpr int N = decltype(NC)::value;
       constexpr int NR = PassNT<T, N>::value;
       using C = Cfg<T, N, NR>;
-      bool persistent = false;
-      if constexpr (kPipeB<T, N>) {
-        if (passb_mode_ == 1) {
+      if constexpr (kLeanB<T, N>) {
+        using L = LeanB32<N>;
+        const tw_t<T>* tw = PassAE<T, N>::value == L::E ? tw_a_ : tw_;
+        static_assert(PassAE<T, N>::value == L::E || Cfg<T, N>::E == L::E, "pass B radix has a twiddle table");
+        if (kxo > gd_.M) {
+          k_passB_lean<N, CFL, true, false><<<dim3(N / 2, nb), L::TPF, L::SMEM, st_>>>(tf, pb, kxo, gd_, inv4, tw,
+                                                                                       enc_base_, batch());
+        } else if (passb_mode_ == 1) {
           // persistent: the autotuned CTA count (about as many as fit at once)
-          persistent = true;
-          constexpr int EP = PipeB<N>::E;
-          static_assert(EP == PassAE<T, N>::value || EP == Cfg<T, N>::E, "pass B radix has a twiddle table");
-          const tw_t<T>* twp = EP == PassAE<T, N>::value ? tw_a_ : tw_;
           const int per_run = std::max(1, std::min(N / 2, (pipeb_grid_ + nb - 1) / nb));
-          auto k = k_passB_pipe<N, CFL>;
-          k<<<dim3(per_run, nb), PipeB<N>::THREADS, PipeB<N>::smem(gd_.M), st_>>>(tf, pb, kxo, gd_, inv4, twp,
-                                                                                    enc_base_, batch());
-          post("k_passB_pipe");
+          k_passB_lean<N, CFL, false, true><<<dim3(per_run, nb), L::TPF, L::SMEM, st_>>>(tf, pb, kxo, gd_, inv4, tw,
+                                                                                         enc_base_, batch());
+        } else {
+          k_passB_lean<N, CFL, false, false><<<dim3(N / 2, nb), L::TPF, L::SMEM, st_>>>(tf, pb, kxo, gd_, inv4, tw,
+                                                                                        enc_base_, batch());
         }
-      }
-      if constexpr (SplitB<T, N>::OK) {
-        if (passb_mode_ == 2) {  // three CTA groups per row pair (small grids)
-          persistent = true;
-          k_passB_split<T, N, CFL><<<dim3(N / NR, nb), SplitB<T, N>::THREADS, SplitB<T, N>::SMEM, st_>>>(
-              tf, pb, kxo, gd_, inv4, tw_, enc_base_, batch());
-          post("k_passB_split");
+        post("k_passB_lean");
+      } else {
+        if constexpr (kPipeB<T, N>) {
+          if (passb_mode_ == 1) {
+            constexpr int EP = PipeB<N>::E;
+            static_assert(EP == PassAE<T, N>::value || EP == Cfg<T, N>::E, "pass B radix has a twiddle table");
+            const tw_t<T>* twp = EP == PassAE<T, N>::value ? tw_a_ : tw_;
+            const int per_run = std::max(1, std::min(N / 2, (pipeb_grid_ + nb - 1) / nb));
+            k_passB_pipe<N, CFL><<<dim3(per_run, nb), PipeB<N>::THREADS, PipeB<N>::smem(gd_.M), st_>>>(
+                tf, pb, kxo, gd_, inv4, twp, enc_base_, batch());
+            post("k_passB_pipe");
+            return;
+          }
         }
-      }
-      if (!persistent) {  // one CTA (group) per row pair; the only form below n = 2048
-        auto k = k_passB<T, N, CFL>;
+        if constexpr (SplitB<T, N>::OK) {
+          if (passb_mode_ == 2) {  // three CTA groups per row pair (small grids)
+            k_passB_split<T, N, CFL><<<dim3(N / NR, nb), SplitB<T, N>::THREADS, SplitB<T, N>::SMEM, st_>>>(
+                tf, pb, kxo, gd_, inv4, tw_, enc_base_, batch());
+            post("k_passB_split");
+            return;
+          }
+        }
+        // one CTA (group) per row pair
         const int g = gb_ ? gb_ : C::G;  // groups per CTA: autotuned
-        const dim3 grid((N / NR + g - 1) / g, nb);
-        // (the rolled form keeps each group's first bracket in shared memory too)
-        const size_t smem = g * (PassSmem<T, N>::GROUP_ELEMS * sizeof(cpx<T>) + (RolledB<T, N>::OK ? N * sizeof(T) : 0));
-        k<<<grid, C::TPF * g, smem, st_>>>(tf, pb, kxo, gd_, inv4, tw_, enc_base_, batch());
+        k_passB<T, N, CFL><<<dim3((N / NR + g - 1) / g, nb), C::TPF * g,
+                             g * PassSmem<T, N>::GROUP_ELEMS * sizeof(cpx<T>), st_>>>(tf, pb, kxo, gd_, inv4, tw_,
+                                                                                      enc_base_, batch());
         post("k_passB");
       }
     });
@@ -1207,6 +1232,13 @@ class EngineT final : public IEngine {
             pb_, c1in, c2in, pbase_[P_PS], pbase_[P_VZ], pbase_[P_FP], pbase_[P_FZ], c1out, c2out, gd_, tab,
             scal_base_, o, tw_, batch(), t5, t6);
         post("k_passC64");
+      } else if constexpr (kLeanC<T, N>) {  // one bracket of a column pair per CTA
+        if (!persistent) {
+          k_passC_lean<N><<<dim3((gd_.M + 1) / 2, nb, 2), LeanC32<N>::TPF, LeanC32<N>::SMEM, st_>>>(
+              pb_, c1in, c2in, pbase_[P_PS], pbase_[P_VZ], pbase_[P_FP], pbase_[P_FZ], c1out, c2out, gd_, d_sc_,
+              scal_base_, o, tw_, batch(), t5, t6);
+          post("k_passC_lean");
+        }
       } else if (!persistent) {  // one CTA (group) per column pair
         auto k = k_passC<T, N>;
         if constexpr (kFuseCA<T, N>) {
@@ -1245,41 +1277,56 @@ class EngineT final : public IEngine {
       set_smem_attr(k_colfft_band2<T, N>, sm);
       if constexpr (RowsCnn<T, N>::OK) set_smem_attr(k_rows_to_cnn8<T, N>, RowsCnn<T, N>::SMEM);
       constexpr size_t smh = PassSmem<T, N>::SMEM;
-      const auto carve = cudaFuncAttributePreferredSharedMemoryCarveout;
       if constexpr (sizeof(T) == 8) {
-        // two CTAs per SM and more
-        cuda_check(cudaFuncSetAttribute(k_passA64<N>, carve, (int)cudaSharedmemCarveoutMaxShared), "carveout");
-        cuda_check(cudaFuncSetAttribute(k_passC64<N>, carve, (int)cudaSharedmemCarveoutMaxShared), "carveout");
+        set_carveout(k_passA64<N>, sm, P64<N>::MINB);
+        set_carveout(k_passC64<N>, Cfg<T, N>::G * kPassC64Group<N>, P64<N>::MINB);
         set_smem_attr(k_passA64<N>, sm);
         set_smem_attr(k_passC64<N>, Cfg<T, N>::G * kPassC64Group<N>);
       } else {
         set_smem_attr(k_passA<T, N>, CfgA<T, N>::SMEM);
-        set_smem_attr(k_passC<T, N>, smh);
+        if constexpr (PassAE<T, N>::value == 16 && N <= 4096)
+          set_carveout(k_passA<T, N>, CfgA<T, N>::SMEM, 512 / CfgA<T, N>::THREADS);
+        if constexpr (!kLeanC<T, N>) set_smem_attr(k_passC<T, N>, smh);
       }
       if constexpr (kAltRadixA<T, N>) set_smem_attr(k_passA<T, N, Cfg<T, N>::E>, CfgAE<T, N, Cfg<T, N>::E>::SMEM);
       if constexpr (sizeof(T) == 8) {
         using B = PassB64<N>;
         constexpr int G = Cfg<T, N>::G;
-        auto attr = [&](auto k, size_t smem) {
-          set_smem_attr(k, smem);
-          cuda_check(cudaFuncSetAttribute(k, carve, (int)cudaSharedmemCarveoutMaxShared), "carveout");
-        };
-        attr(k_passB64<N, true, false>, G * B::GROUP);
-        attr(k_passB64<N, false, false>, G * B::GROUP);
-        attr(k_passB64<N, false, true>, G * B::GROUP);
-        if constexpr (SplitB64<N>::OK) {
-          attr(k_passB64_split<N, true>, SplitB64<N>::SMEM);
-          attr(k_passB64_split<N, false>, SplitB64<N>::SMEM);
+        for (auto k : {k_passB64<N, true, false>, k_passB64<N, false, false>, k_passB64<N, false, true>}) {
+          set_smem_attr(k, G * B::GROUP);
+          set_carveout(k, G * B::GROUP, P64<N>::MINB);
         }
+        if constexpr (SplitB64<N>::OK) {
+          set_smem_attr(k_passB64_split<N, true>, SplitB64<N>::SMEM);
+          set_smem_attr(k_passB64_split<N, false>, SplitB64<N>::SMEM);
+        }
+      } else if constexpr (kLeanB<T, N>) {
+        using L = LeanB32<N>;
+        for (auto k : {k_passB_lean<N, true, false, false>, k_passB_lean<N, false, false, false>,
+                       k_passB_lean<N, true, false, true>, k_passB_lean<N, false, false, true>,
+                       k_passB_lean<N, false, true, false>}) {
+          set_smem_attr(k, L::SMEM);
+          set_carveout(k, L::SMEM, L::MINB);
+        }
+        int per_sm = 0;
+        cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_passB_lean<N, false, false, true>, L::TPF,
+                                                                 L::SMEM),
+                   "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+        if (per_sm < 1) throw Error(kEINVAL, "pass B does not fit on this device");
+        pipeb_ctas_ = per_sm * sms_;
       } else {
-        set_smem_attr(k_passB<T, N, true>, RolledB<T, N>::SMEM);
-        set_smem_attr(k_passB<T, N, false>, RolledB<T, N>::SMEM);
+        set_smem_attr(k_passB<T, N, true>, smh);
+        set_smem_attr(k_passB<T, N, false>, smh);
       }
       if constexpr (sizeof(T) == 4 && SplitB<T, N>::OK) {
         set_smem_attr(k_passB_split<T, N, true>, SplitB<T, N>::SMEM);
         set_smem_attr(k_passB_split<T, N, false>, SplitB<T, N>::SMEM);
       }
       if constexpr (kFuseCA<T, N>) set_smem_attr(k_passC<T, N, true>, smh);
+      if constexpr (kLeanC<T, N>) {
+        set_smem_attr(k_passC_lean<N>, LeanC32<N>::SMEM);
+        set_carveout(k_passC_lean<N>, LeanC32<N>::SMEM, LeanC32<N>::MINB);
+      }
       if constexpr (kPipeC<T, N>) {
         set_smem_attr(k_passC_pipe<N>, PipeC<N>::SMEM);
         cuda_check(cudaFuncSetAttribute(k_passC_pipe<N>, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1417,7 +1464,7 @@ class EngineT final : public IEngine {
       {
         std::vector<std::pair<int, int>> cands;
         for (int g = GB; g >= 1; g /= 2) cands.push_back({0, g});
-        if constexpr (kPipeB<T, N>) {
+        if constexpr (kPipeB<T, N> || kLeanB<T, N>) {
           cands.push_back({1, pipeb_ctas_});
           if (pipeb_ctas_ >= 2 * sms) cands.push_back({1, pipeb_ctas_ / 2});
         }
@@ -1444,6 +1491,7 @@ class EngineT final : public IEngine {
         std::vector<CandC> cands;
         for (int g = GB; g >= 1; g /= 2) {
           cands.push_back({0, g, 1, 1});
+          if constexpr (kLeanC<T, N>) break;  // its launch shape is fixed
           if constexpr (kChunkC<T, N>) {
             cands.push_back({0, g, 2, 1});
             // teams of 2 or 4 groups per column pair share its update
@@ -1461,7 +1509,7 @@ class EngineT final : public IEngine {
         cpx<T>* c4 = planes_[P_C4];
         const std::vector<float> us = time_candidates(cands.size(), [&](size_t i) {
           passc_mode_ = cands[i].mode;
-          pipec_grid_ = cands[i].mode ? cands[i].grid : 0;
+          pipec_grid_ = cands[i].mode == 1 ? cands[i].grid : 0;
           gc_ = cands[i].mode ? GB : cands[i].grid;
           fc_ = cands[i].chunks;
           wc_ = cands[i].wide;
@@ -1638,7 +1686,7 @@ class EngineT final : public IEngine {
     snprintf(b, sizeof b,
              "], \"chosen_c\": \"%s\", \"ctas_c\": %d, \"groups_c\": %d, \"chunks_c\": %d, \"team_c\": %d, "
              "\"fused_ca\": %s}",
-             passc_mode_ ? "persistent" : "per_column_pair", passc_mode_ ? pipec_grid_ : 0, gc_, fc_, wc_,
+             passc_mode_ ? "persistent" : "per_column_pair", passc_mode_ == 1 ? pipec_grid_ : 0, gc_, fc_, wc_,
              fuse_ca() ? "true" : "false");
     return r + b;
   }

@@ -186,7 +186,16 @@ struct BlockFFT {
   }
   static constexpr int TW_ELEMS = tw_off(NST) > 0 ? tw_off(NST) : 1;
 
-  template <int DIR, int S, int NS>
+  // Position of value i of a buffer of N float2 (HALF: both transforms' real
+  // parts, then their imaginary parts go through it; half the shared memory,
+  // twice the barriers): free of bank conflicts in every stage of radix 8.
+  static __device__ __forceinline__ int pos8(int i) { return i ^ ((i >> LOGE) & 15); }
+  static __device__ __forceinline__ int pos8(int lane, int q) {  // of value lane + q TPF
+    if constexpr (TPF % (16 << LOGE) == 0) return pos8(lane) + q * TPF;
+    else return pos8(lane + q * TPF);
+  }
+
+  template <int DIR, int S, int NS, bool HALF = false>
   static __device__ __forceinline__ void stage(cpx<T> (&v)[NT][E], int lane, cpx<T>* sm,
                                                const tw_t<T>* __restrict__ tw) {
     constexpr int R = (S == NST - 1) ? LAST_R : E;
@@ -215,7 +224,30 @@ struct BlockFFT {
         for (int r = 0; r < R; ++r) v[t][m + r * B] = u[r];
       }
     }
-    if constexpr (S < NST - 1) {
+    if constexpr (S < NST - 1 && HALF) {
+      static_assert(!HALF || NT == 2, "two transforms a position");
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+#pragma unroll
+        for (int m = 0; m < B; ++m) {
+          const int j = lane + m * TPF;
+          const int base = ((j >> LOGNS) << (LOGNS + ilog2(R))) + (j & (NS - 1));
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+            sm[pos8(base + r * NS)] = h ? mkc<T>(v[0][m + r * B].y, v[NT - 1][m + r * B].y)
+                                        : mkc<T>(v[0][m + r * B].x, v[NT - 1][m + r * B].x);
+        }
+        fft_sync<TPF>();
+#pragma unroll
+        for (int q = 0; q < E; ++q) {
+          const cpx<T> w = sm[pos8(lane, q)];
+          (h ? v[0][q].y : v[0][q].x) = w.x;
+          (h ? v[NT - 1][q].y : v[NT - 1][q].x) = w.y;
+        }
+        fft_sync<TPF>();
+      }
+      stage<DIR, S + 1, NS * R, HALF>(v, lane, sm, tw);
+    } else if constexpr (S < NST - 1) {
 #pragma unroll
       for (int m = 0; m < B; ++m) {
         const int j = lane + m * TPF;
@@ -243,15 +275,15 @@ struct BlockFFT {
         }
       }
       fft_sync<TPF>();
-      stage<DIR, S + 1, NS * R>(v, lane, sm, tw);
+      stage<DIR, S + 1, NS * R, HALF>(v, lane, sm, tw);
     }
   }
 
   // X_t[k] = sum_x x_t[x] exp(DIR*2*pi*i*x*k/N), unnormalised, t < NT.
-  template <int DIR>
+  template <int DIR, bool HALF = false>
   static __device__ __forceinline__ void run(cpx<T> (&v)[NT][E], int lane, cpx<T>* sm,
                                              const tw_t<T>* __restrict__ tw) {
-    stage<DIR, 0, 1>(v, lane, sm, tw);
+    stage<DIR, 0, 1, HALF>(v, lane, sm, tw);
   }
 
   // Natural-order result to shared memory so that any thread of the group can

@@ -64,13 +64,12 @@ struct Cfg {
 };
 
 // Transforms carried at once by one group in passes A, B and C.  Two in the
-// FP32 path up to n = 4096 ("tiled" mode): pass A and C transform two
-// adjacent kx columns, pass B two adjacent rows, and the mixed planes use the
-// pair-tiled layout below so that every access moves whole 32-byte sectors.
-// One at n = 8192 (plain column layout T[kx][y]) and in the FP64 path, which
-// has passes of its own (r2d3c_pass64.cuh).
+// FP32 path: pass A and C transform two adjacent kx columns, pass B two
+// adjacent rows, and the mixed planes use the pair-tiled layout below so that
+// every access moves whole 32-byte sectors.  One in the FP64 path, which has
+// passes of its own (r2d3c_pass64.cuh).
 template <typename T, int N> struct PassNT {
-  static constexpr int value = (sizeof(T) == 4 && N <= 4096) ? 2 : 1;
+  static constexpr int value = sizeof(T) == 4 ? 2 : 1;
 };
 
 // Elements per thread of pass A: radix-16 (up to 255 registers, fewer
@@ -100,7 +99,6 @@ struct PassSmem {
   static constexpr int NT = PassNT<T, N>::value;
   using C = Cfg<T, N, NT>;
   static constexpr size_t HOLD_BYTES = (size_t)NT * N * sizeof(cpx<T>);
-  static_assert(sizeof(T) == 8 || C::FFT::SMEM_BYTES + HOLD_BYTES <= 200 * 1024, "fits an SM");
   static constexpr size_t GROUP_ELEMS = (size_t)NT * C::FFT::SMEM_ELEMS + (size_t)NT * N;
   static constexpr size_t SMEM = (size_t)C::G * GROUP_ELEMS * sizeof(cpx<T>);
 };
@@ -330,7 +328,7 @@ k_passA(const cpx<T>* __restrict__ ps, const cpx<T>* __restrict__ vz, cpx<T>* __
   auto src_at = [&](const cpx<T>* sp, int t, int q) -> cpx<T> {
     const int col = kx0 + t, ky = kyi[q];
     const bool in = col < gd.M && (ky <= gd.L && -ky <= gd.L) && col * col + ky * ky <= gd.kmaxi;
-    return in ? sp[(size_t)col * N + lane + q * C::TPF] : czero<T>();
+    return in ? __ldcg(&sp[(size_t)col * N + lane + q * C::TPF]) : czero<T>();
   };
 #pragma unroll 1
   for (int f = f0; f < f0 + fpc; ++f) {
@@ -453,18 +451,6 @@ __device__ __forceinline__ void cfl_max_sq(const cpx<T> (&v)[NT][E], unsigned lo
   if ((threadIdx.x & 31) == 0) atomicMax(enc, enc_ordered((double)m));
 }
 
-// Pass B with one rolled copy of the transform code (a loop over the four
-// transforms that is not unrolled) and the first bracket p1 in shared
-// memory, for the FP32 grid with one row per group (n = 8192): unrolled,
-// the compiler interleaves the four 8192-point transforms and spills
-// hundreds of bytes per thread.  The forward transform is the inverse one
-// of the conjugate, conjugated: bit-identical to the unrolled form.
-template <typename T, int N>
-struct RolledB {
-  static constexpr bool OK = sizeof(T) == 4 && PassNT<T, N>::value == 1;
-  static constexpr size_t SMEM = PassSmem<T, N>::SMEM + (OK ? (size_t)Cfg<T, N, 1>::G * N * sizeof(T) : 0);
-};
-
 template <typename T, int N, bool CFL>
 __global__ void __launch_bounds__(Cfg<T, N, PassNT<T, N>::value>::THREADS, 1)
 k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid gd, T inv_n4,
@@ -487,46 +473,6 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
   const int M = gd.M;
   const size_t plane = (size_t)M * N;
   cpx<T> v[NR][C::E];
-  if constexpr (RolledB<T, N>::OK) {
-    T* P1 = reinterpret_cast<T*>(smbase_ + (size_t)(blockDim.x / C::TPF) * PS::GROUP_ELEMS) + (size_t)g * N;
-#pragma unroll 1
-    for (int f = 0; f < 4; ++f) {
-      if (f < 3) {
-        const cpx<T>* pa = tf + (size_t)(2 * f) * plane;
-#pragma unroll
-        for (int q = 0; q < C::E; ++q) {
-          cpx<T> z[1];
-          packed_pair<T, N, 1>(pa, pa + plane, lane + q * C::TPF, y0, M, z);
-          v[0][q] = z[0];
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < C::E; ++q) v[0][q].y = -v[0][q].y;
-      }
-      F::template run<+1>(v, lane, sm, tw);
-      // each thread reads back only the positions it wrote: no barrier needed
-      if (f == 0) {
-        if constexpr (CFL) cfl_max_sq<T, 1, C::E>(v, cfl_enc);
-#pragma unroll
-        for (int q = 0; q < C::E; ++q) hold[lane + q * C::TPF] = v[0][q];
-      } else if (f == 1) {
-#pragma unroll
-        for (int q = 0; q < C::E; ++q) {
-          const cpx<T> a = hold[lane + q * C::TPF];
-          P1[lane + q * C::TPF] = (a.x * v[0][q].y - a.y * v[0][q].x) * inv_n4;
-        }
-      } else if (f == 2) {
-#pragma unroll
-        for (int q = 0; q < C::E; ++q) {
-          const cpx<T> a = hold[lane + q * C::TPF];
-          v[0][q] = mkc<T>(P1[lane + q * C::TPF], (a.x * v[0][q].y - a.y * v[0][q].x) * inv_n4);
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < C::E; ++q) v[0][q].y = -v[0][q].y;
-      }
-    }
-  } else {
   T p1[NR][C::E];
   // pair (d_x psi, d_y psi)
 #pragma unroll
@@ -578,7 +524,6 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
     }
   // forward x-FFT of both real products at once
   F::template run<-1>(v, lane, sm, tw);
-  }
   F::to_smem(v, lane, sm);
   fft_sync<C::TPF>();
   const size_t oplane = (size_t)gd.nh * N;
@@ -775,8 +720,7 @@ struct PipeB {
 
 // pass B runs as k_passB_pipe where it applies
 template <typename T, int N>
-constexpr bool kPipeB = sizeof(T) == 4 && PassNT<T, N>::value == 2 && PipeB<N>::THREADS >= 64 &&
-                        PipeB<N>::THREADS <= 512;
+constexpr bool kPipeB = sizeof(T) == 4 && PipeB<N>::THREADS >= 64 && N <= 1024;
 
 // Row t (0/1) of the staged pair at column kk: S holds float4 (row 0, row 1).
 __device__ __forceinline__ float2 staged_row(const float4* S, int idx, int t) {
@@ -998,7 +942,8 @@ __device__ __forceinline__ void prefetch_columns_l2(const cpx<T>* p, int ncol, i
 // 16-byte loads and stores), two row pairs per iteration with all loads of
 // an iteration issued before its stores.  Each element is loaded and stored
 // by one thread.  Every thread of the CTA calls it (one barrier inside).
-template <typename T, int N, int NT, int E, int TPF>
+// (CHUNK: the chunk where the caller knows it at compile time, else -2)
+template <typename T, int N, int NT, int E, int TPF, int CHUNK = -2>
 __device__ __forceinline__ void passC_update_pairs(cpx<T>* sm, const cpx<T>* hold, const cpx<T> (&v)[NT][E],
                                                    int lane, int kx0, const cpx<T>* c1in, const cpx<T>* c2in,
                                                    const cpx<T>* ps, const cpx<T>* vz, const cpx<T>* __restrict__ fp,
@@ -1012,7 +957,7 @@ __device__ __forceinline__ void passC_update_pairs(cpx<T>* sm, const cpx<T>* hol
   // over ustride threads (thread uidx; default: the group's own TPF), of
   // which the owner group's results are in sm / hold.
   if (uidx < 0) uidx = lane;
-  const bool do1 = chunk != 1, do2 = chunk != 0;
+  const bool do1 = CHUNK == -2 ? chunk != 1 : CHUNK != 1, do2 = CHUNK == -2 ? chunk != 0 : CHUNK != 0;
   cpx<T>* c6s = sm;
   if (do2 && owner) {
 #pragma unroll
@@ -1315,8 +1260,7 @@ template <typename T, int N>
 constexpr bool kFuseCA = sizeof(T) == 4 && N <= 512 && PassNT<T, N>::value == 2 &&
                          !kAltRadixA<T, N> && PassAE<T, N>::value == Cfg<T, N>::E;
 template <typename T, int N>
-constexpr bool kPipeC = sizeof(T) == 4 && PassNT<T, N>::value == 2 &&
-                        PipeC<N>::THREADS >= 64 && PipeC<N>::THREADS <= 512;
+constexpr bool kPipeC = sizeof(T) == 4 && PipeC<N>::THREADS >= 64 && N <= 4096;
 
 template <int N>
 __global__ void __launch_bounds__(PipeC<N>::THREADS, PipeC<N>::MINB)

@@ -78,7 +78,7 @@ k_passA64(const double2* __restrict__ ps, const double2* __restrict__ vz, double
       if (P::dead(q)) continue;
       const int ky = ky_of(lane + q * TPF, N), k2 = kx * kx + ky * ky;
       const bool in = kx < gd.M && (ky <= gd.L && -ky <= gd.L) && k2 <= gd.kmaxi;
-      x[q] = in ? sp[lane + q * TPF] : czero<T>();
+      x[q] = in ? __ldcg(sp + lane + q * TPF) : czero<T>();
       if (mult(q) == 0) {  // 0 times a finite value: no part in the vector's scale
         if (fx_upper(x[q].x) < 0x7ff00000u) x[q].x = 0.0;
         if (fx_upper(x[q].y) < 0x7ff00000u) x[q].y = 0.0;
@@ -169,8 +169,8 @@ struct PassB64 {
     for (int q = 0; q < KQ; ++q) {
       const int kx = lane + q * TPF;
       const size_t i = mix_idx<N, 2>(kx < M ? kx : 0, y, M);
-      a[q] = kx < M ? pa[i] : make_double2(0.0, 0.0);
-      b[q] = kx < M ? pb[i] : make_double2(0.0, 0.0);
+      a[q] = kx < M ? __ldcg(pa + i) : make_double2(0.0, 0.0);
+      b[q] = kx < M ? __ldcg(pb + i) : make_double2(0.0, 0.0);
       if (kx == 0) a[q].y = b[q].y = 0.0;  // Im of the kx = 0 column is ignored
       mh = max(mh, max(max(fx_upper(a[q].x), fx_upper(a[q].y)), max(fx_upper(b[q].x), fx_upper(b[q].y))));
       lo |= __double2loint(a[q].x) | __double2loint(a[q].y) | __double2loint(b[q].x) | __double2loint(b[q].y);
@@ -339,6 +339,9 @@ k_passB64(double2* tf, double2* __restrict__ pb, int kxo, DevGrid gd, const int4
     return tf + (size_t)(j < gd.M ? 2 : 3) * plane + mix_idx<N, 2>(j < gd.M ? j : j - gd.M, y, gd.M);
   };
   int e1 = 0, k1 = 0, kb1 = 0, kb2 = 0;
+  // the later planes' rows (both of the pair's) into L2 while the first
+  // transform runs
+  if (lane0 < 4 && !(y & 1)) prefetch_l2(tf + (size_t)(2 + lane0) * plane + (size_t)(y >> 1) * gd.M * 2, (size_t)2 * gd.M);
 #pragma unroll 1
   for (int f = 0; f < 3; ++f) {
     // the transform's addresses are derived from an opaque lane index every
@@ -377,7 +380,7 @@ k_passB64(double2* tf, double2* __restrict__ pb, int kxo, DevGrid gd, const int4
   double p1[E], p2[E];
 #pragma unroll
   for (int q = 0; q < E; q += 2) {
-    const double2 p = *slot(lane, q);
+    const double2 p = __ldcg(slot(lane, q));
     p1[q] = p.x;
     p1[q + 1] = p.y;
   }
@@ -521,7 +524,7 @@ k_passC64(const double2* __restrict__ pb, const double2* c1in, const double2* c2
     double2 v[E];
     const double2* src = pb + blockIdx.y * bs.pb + (second ? (size_t)gd.nh * N : 0) + mix_idx<N, 2>(ok ? kx : 0, lane, gd.nh);
 #pragma unroll
-    for (int q = 0; q < E; ++q) v[q] = src[(size_t)q * TPF * gd.nh];
+    for (int q = 0; q < E; ++q) v[q] = __ldcg(src + (size_t)q * TPF * gd.nh);
     int e, s;
     F::scale(v, lane, reinterpret_cast<int4*>(sm + F::RED), e, s);
     fx u[E];
@@ -553,9 +556,9 @@ k_passC64(const double2* __restrict__ pb, const double2* c1in, const double2* c2
       const int q = i0 + b < LO ? i0 + b : i0 + b + E - LIVE;
       const int j = lane + q * TPF, ky = ky_of(j, N), k2 = kx * kx + ky * ky, ay = ky < 0 ? -ky : ky;
       if (ay <= gd.L && k2 <= gd.kmaxi && k2 >= 1) {
-        a[b] = other[j];
-        p[b] = base[j];
-        f[b] = force[j];
+        a[b] = __ldcg(other + j);
+        p[b] = __ldcg(base + j);
+        f[b] = __ldcg(force + j);
         d[b] = dt[ay];
         w[b] = wk[ay];
         if (!second) i2[b] = ik2t[ay];
