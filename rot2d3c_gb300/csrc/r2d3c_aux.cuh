@@ -124,11 +124,59 @@ constexpr int kMaxTerms = 24;
 struct SumTerm {
   int kind, ia, ib, kin;
 };
+// The terms of one pass, sorted out on the host (plan_sums): the distinct
+// products (|a|^2, Re(b conj a), Re(d_y b conj a)) and the distinct powers of
+// ka2 are formed once per element, and a term is one multiply-add of the two.
+// (Formed term by term, with a division for every negative power, the 22
+// terms of cond_check took some 250 FP64 operations an element: 703 us at
+// 2048^2 instead of 353, now bound by the FP64 pipe with some 70.)
+constexpr int kMaxProd = 12, kMaxPow = 16;
+enum SumWhere : int { W_ALL = 0, W_NONZERO = 1, W_DISC = 2, W_BAND = 4 };
 struct SumList {
-  int nterms;
-  SumTerm t[kMaxTerms];
+  int nterms, nprod, npow;
+  struct {
+    short prod, pow, where;
+  } t[kMaxTerms];
+  struct {
+    short ia, ib, dy;  // ia == ib and dy == 0: |a|^2
+  } prod[kMaxProd];
+  int kin[kMaxPow];
   double band_lo, band_hi;
 };
+inline bool plan_sums(int nterms, const SumTerm* in, double band_lo, double band_hi, SumList& sl) {
+  sl = SumList{};
+  sl.nterms = nterms;
+  sl.band_lo = band_lo;
+  sl.band_hi = band_hi;
+  for (int i = 0; i < nterms; ++i) {
+    const SumTerm& m = in[i];
+    const bool energy = m.kind == S_ENERGY || m.kind == S_BAND_KA2 || m.kind == S_BAND;
+    const int ib = energy ? m.ia : m.ib, dy = m.kind == S_INERPROD_DY;
+    const int kin = m.kind == S_BAND_KA2 ? 1 : m.kind == S_ENERGY || m.kind == S_INERPROD ? m.kin : 0;
+    int p = 0, k = 0;
+    while (p < sl.nprod && !(sl.prod[p].ia == m.ia && sl.prod[p].ib == ib && sl.prod[p].dy == dy)) ++p;
+    while (k < sl.npow && sl.kin[k] != kin) ++k;
+    if (p == kMaxProd || k == kMaxPow) return false;
+    if (p == sl.nprod) {
+      sl.prod[p].ia = (short)m.ia;
+      sl.prod[p].ib = (short)ib;
+      sl.prod[p].dy = (short)dy;
+      ++sl.nprod;
+    }
+    if (k == sl.npow) sl.kin[sl.npow++] = kin;
+    sl.t[i].prod = (short)p;
+    sl.t[i].pow = (short)k;
+    sl.t[i].where = (short)(energy && m.kind != S_ENERGY ? W_BAND
+                            : (m.kind == S_ENERGY ? 0 : W_DISC) | (kin < 0 ? W_NONZERO : 0));
+  }
+  return true;
+}
+
+// (double)i for 0 <= i < 2^31 by one addition (the conversion takes more than
+// four times as long on the FP64 pipe)
+__device__ __forceinline__ double int_to_double(int i) {
+  return __hiloint2double(0x43300000, i) - 4503599627370496.0;
+}
 
 constexpr int kSumThreads = 256;
 
@@ -142,14 +190,15 @@ k_halfplane_sums(const cpx<T>* __restrict__ p0, const cpx<T>* __restrict__ p1,
   for (int t = 0; t < kMaxTerms; ++t) acc[t] = 0.0;
   const cpx<T>* planes[4] = {p0, p1, p2, p3};
   const size_t total = (size_t)gd.nh * gd.n;
+  bool neg = false;
+  for (int k = 0; k < sl.npow; ++k) neg |= sl.kin[k] < 0;
   for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
        idx += (size_t)gridDim.x * blockDim.x) {
     int i, j;
     plane_ij(idx, gd.n, i, j);
     const int kx = kx_of(i, gd.n), ky = ky_of(j, gd.n);
     const int k2 = kx * kx + ky * ky;
-    const double ka2 = (double)k2;
-    const double two = i == 0 ? 1.0 : 2.0;
+    const double ka2 = int_to_double(k2);
     cpx<double> v[4];
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
@@ -160,34 +209,29 @@ k_halfplane_sums(const cpx<T>* __restrict__ p0, const cpx<T>* __restrict__ p1,
         v[p] = mkc<double>(0.0, 0.0);
       }
     }
+    double prod[kMaxProd], pw[kMaxPow];
+    for (int p = 0; p < sl.nprod; ++p) {
+      const cpx<double> a = v[sl.prod[p].ia];
+      cpx<double> b = v[sl.prod[p].ib];
+      if (sl.prod[p].dy) {
+        const double k = ky < 0 ? -int_to_double(-ky) : int_to_double(ky);
+        b = mkc<double>(-k * b.y, k * b.x);
+      }
+      const double r = b.x * a.x + b.y * a.y;
+      prod[p] = i == 0 ? r : r + r;  // two = 1 on the kx = 0 column
+    }
+    const double inv = neg && k2 >= 1 ? 1.0 / ka2 : 0.0;
+    for (int k = 0; k < sl.npow; ++k) {
+      const int e = sl.kin[k];
+      pw[k] = e == 0 ? 1.0 : e > 0 ? powi(ka2, e) : powi(inv, -e);
+    }
+    int where = (k2 >= 1 ? W_NONZERO : 0) | (k2 <= gd.kmaxi ? W_DISC : 0);
+    if (ka2 <= sl.band_hi && ka2 >= sl.band_lo) where |= W_BAND;
 #pragma unroll
     for (int t = 0; t < kMaxTerms; ++t) {
       if (t >= sl.nterms) break;
-      const SumTerm tm = sl.t[t];
-      const cpx<double> a = v[tm.ia], b = v[tm.ib];
-      double val = 0.0;
-      switch (tm.kind) {
-        case S_ENERGY:
-          if (tm.kin >= 0 || k2 >= 1) val = two * (a.x * a.x + a.y * a.y) * powi(ka2, tm.kin);
-          break;
-        case S_INERPROD:
-          if (k2 <= gd.kmaxi && (tm.kin >= 0 || k2 >= 1))
-            val = two * powi(ka2, tm.kin) * (b.x * a.x + b.y * a.y);
-          break;
-        case S_INERPROD_DY:
-          if (k2 <= gd.kmaxi) {
-            const double dx = -(double)ky * b.y, dy = (double)ky * b.x;
-            val = two * (dx * a.x + dy * a.y);
-          }
-          break;
-        case S_BAND_KA2:
-          if (ka2 <= sl.band_hi && ka2 >= sl.band_lo) val = two * ka2 * (a.x * a.x + a.y * a.y);
-          break;
-        default:  // S_BAND
-          if (ka2 <= sl.band_hi && ka2 >= sl.band_lo) val = two * (a.x * a.x + a.y * a.y);
-          break;
-      }
-      acc[t] += val;
+      const int w = sl.t[t].where;
+      if ((where & w) == w) acc[t] = fma(prod[sl.t[t].prod], pw[sl.t[t].pow], acc[t]);
     }
   }
   __shared__ double red[kSumThreads];
@@ -209,6 +253,8 @@ static __global__ void k_finalize_sums(const double* __restrict__ partials, int 
   const int t = threadIdx.x;
   if (t >= nterms) return;
   double s = 0.0;
+  // (the loads of 38 partials in flight together)
+#pragma unroll 38
   for (int b = 0; b < nblocks; ++b) s += partials[(size_t)b * kMaxTerms + t];
   out[t] = s * scale;
 }
@@ -218,14 +264,20 @@ static __global__ void k_finalize_sums(const double* __restrict__ partials, int 
 // kmn = int(sqrt(ka2)+.5) == b  <=>  (2b-1)^2 < 4 ka2 < (2b+1)^2.
 // out[(b-1)*5 + {0..4}] = Ek, Ezk, Fl0, Fl1, Fl2 (times 1/n^4).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ long long isqrt_ll(long long v) {
-  if (v <= 0) return 0;
-  long long r = (long long)sqrt((double)v);
-  while (r * r > v) --r;
-  while ((r + 1) * (r + 1) <= v) ++r;
+// floor(sqrt(v)), 0 <= v < 2^30: the FP32 root (less than 2^-8 off) and one
+// correction either way
+__device__ __forceinline__ int isqrt_small(int v) {
+  int r = (int)sqrtf((float)v);
+  if (r * r > v) --r;
+  if ((r + 1) * (r + 1) <= v) ++r;
   return r;
 }
 
+// A shell is two elements or three thick wherever it is crossed along its
+// steeper direction: for |ky| > kx a thread takes one kx and the shell's few
+// |ky|, for |ky| <= kx one |ky| and its few kx.  (One warp per kx, most of its
+// lanes without an element and each with two FP64 square roots, took 1659 us
+// at 2048^2 instead of 93.)  4 ka2 < 2^28 at n = 8192: 32-bit integers throughout.
 constexpr int kShellThreads = 256;
 
 template <typename T>
@@ -234,54 +286,38 @@ k_shells(const cpx<T>* __restrict__ ps, const cpx<T>* __restrict__ vz,
          const cpx<T>* __restrict__ c2, const cpx<T>* __restrict__ c1, DevGrid gd, double scale,
          double* __restrict__ out) {
   const int b = blockIdx.x + 1;
-  const int n = gd.n;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int NW = kShellThreads / 32;
+  const int n = gd.n, half = n / 2;
   double acc[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  const long long lo = (long long)(2 * b - 1) * (2 * b - 1);
-  const long long hi = (long long)(2 * b + 1) * (2 * b + 1);
-  const int kxmax = min(b, n / 2);
-  for (int kx = warp; kx <= kxmax; kx += NW) {
-    const long long l2 = lo - 4LL * kx * kx;  // need 4 ky^2 > l2
-    const long long h2 = hi - 4LL * kx * kx;  // need 4 ky^2 < h2
-    if (h2 <= 0) continue;
-    long long kmin = 0;
-    if (l2 >= 0) {
-      kmin = isqrt_ll(l2 / 4);
-      while (4 * kmin * kmin <= l2) ++kmin;
-    }
-    long long kmaxk = isqrt_ll(h2 / 4) + 1;
-    while (kmaxk >= 0 && 4 * kmaxk * kmaxk >= h2) --kmaxk;
-    if (kmaxk < kmin) continue;
+  const int lo = (2 * b - 1) * (2 * b - 1), hi = (2 * b + 1) * (2 * b + 1);
+  auto add = [&](int kx, int j, int k2) {
+    const size_t idx = (size_t)kx * n + j;
     const double two = kx == 0 ? 1.0 : 2.0;
-    const double ka2c = (double)kx * kx;
-    // positive ky in [kmin, min(kmaxk, n/2-1)], negative ky in
-    // [-min(kmaxk, n/2), -max(kmin,1)]
-    for (int side = 0; side < 2; ++side) {
-      long long a0, a1;
-      if (side == 0) {
-        a0 = kmin;
-        a1 = min(kmaxk, (long long)(n / 2 - 1));
-      } else {
-        a0 = max(kmin, 1LL);
-        a1 = min(kmaxk, (long long)(n / 2));
-      }
-      for (long long k = a0 + lane; k <= a1; k += 32) {
-        const int j = side == 0 ? (int)k : (int)(n - k);
-        const size_t idx = (size_t)kx * n + j;
-        const double ka2 = ka2c + (double)(k * k);
-        const cpx<T> p = ps[idx], z = vz[idx];
-        const double pe = (double)p.x * p.x + (double)p.y * p.y;
-        acc[0] += two * ka2 * pe;
-        acc[1] += two * ((double)z.x * z.x + (double)z.y * z.y);
-        if (c2) {
-          const cpx<T> q2 = c2[idx], q1 = c1[idx];
-          const double r2 = (double)p.x * q2.x + (double)p.y * q2.y;
-          acc[2] += two * ka2 * r2;
-          acc[3] += two * r2;
-          acc[4] -= two * ((double)z.x * q1.x + (double)z.y * q1.y);
-        }
-      }
+    const double w = int_to_double(kx == 0 ? k2 : 2 * k2);
+    const cpx<T> p = ps[idx], z = vz[idx];
+    acc[0] = fma(w, fma((double)p.x, (double)p.x, (double)p.y * p.y), acc[0]);
+    acc[1] = fma(two, fma((double)z.x, (double)z.x, (double)z.y * z.y), acc[1]);
+    if (c2) {
+      const cpx<T> q2 = c2[idx], q1 = c1[idx];
+      const double r2 = fma((double)p.x, (double)q2.x, (double)p.y * q2.y);
+      acc[2] = fma(w, r2, acc[2]);
+      acc[3] = fma(two, r2, acc[3]);
+      acc[4] = fma(-two, fma((double)z.x, (double)q1.x, (double)z.y * q1.y), acc[4]);
+    }
+  };
+  const int amax = min(b, half);
+  for (int a = threadIdx.x; a <= amax; a += kShellThreads) {
+    const int l2 = lo - 4 * a * a, h2 = hi - 4 * a * a;  // l2 < 4 c^2 < h2
+    if (h2 <= 0) continue;
+    const int cmin = l2 < 0 ? 0 : isqrt_small(l2 >> 2) + 1, cmax = min(isqrt_small((h2 - 1) >> 2), half);
+    for (int c = max(cmin, a + 1); c <= cmax; ++c) {  // kx = a, |ky| = c > kx
+      const int k2 = a * a + c * c;
+      if (c < half) add(a, c, k2);
+      add(a, n - c, k2);
+    }
+    for (int c = max(cmin, a); c <= cmax; ++c) {  // |ky| = a, kx = c >= |ky|
+      const int k2 = a * a + c * c;
+      if (a < half) add(c, a, k2);
+      if (a > 0) add(c, n - a, k2);
     }
   }
   __shared__ double red[kShellThreads];
@@ -556,7 +592,7 @@ __global__ void k_shell_weight2(const cpx<T>* a_in, const cpx<T>* b_in, cpx<T>* 
     plane_ij(i, gd.n, kx, j);
     const int ky = ky_of(j, gd.n);
     // (2b-1)^2 < 4 ka2 < (2b+1)^2  <=>  b = (isqrt(4 ka2) + 1) / 2
-    const int bsh = (int)((isqrt_ll(4LL * ((long long)kx * kx + (long long)ky * ky)) + 1) / 2);
+    const int bsh = (isqrt_small(4 * (kx * kx + ky * ky)) + 1) / 2;
     const T fa = bsh < nw ? (T)w[bsh] : (T)0;
     const T fb = bsh < nw ? (T)w[nw + bsh] : (T)0;
     a[i] = mkc<T>(u.x * fa, u.y * fa);
@@ -592,7 +628,7 @@ k_colfft_band2(const cpx<T>* __restrict__ in, cpx<T>* __restrict__ a, cpx<T>* __
 #pragma unroll
     for (int q = 0; q < C::E; ++q) {
       const int j = lane + q * C::TPF, ky = ky_of(j, N);
-      const int bsh = (int)((isqrt_ll(4LL * ((long long)kx * kx + (long long)ky * ky)) + 1) / 2);
+      const int bsh = (isqrt_small(4 * (kx * kx + ky * ky)) + 1) / 2;
       const T f = bsh < nw ? (T)wp[bsh] : (T)0;
       dst[j] = mkc<T>(v[0][q].x * f, v[0][q].y * f);
     }

@@ -280,12 +280,10 @@ class EngineT final : public IEngine {
   void enqueue_sums(int nterms, const int* kind, const int* ia, const int* ib, const int* kin,
                     double band_lo, double band_hi, const int* planes4) {
     if (nterms < 1 || nterms > kMaxTerms) throw Error(kEINVAL, "bad number of sum terms");
+    SumTerm in[kMaxTerms];
+    for (int t = 0; t < nterms; ++t) in[t] = SumTerm{kind[t], ia[t], ib[t], kin[t]};
     SumList sl;
-    std::memset(&sl, 0, sizeof(sl));
-    sl.nterms = nterms;
-    for (int t = 0; t < nterms; ++t) sl.t[t] = SumTerm{kind[t], ia[t], ib[t], kin[t]};
-    sl.band_lo = band_lo;
-    sl.band_hi = band_hi;
+    if (!plan_sums(nterms, in, band_lo, band_hi, sl)) throw Error(kEINVAL, "too many distinct sum terms");
     const cpx<T>* p[4];
     for (int i = 0; i < 4; ++i) p[i] = planes4[i] >= 0 ? planes_[planes4[i]] : nullptr;
     k_halfplane_sums<T><<<kSumBlocks, kSumThreads, 0, st_>>>(p[0], p[1], p[2], p[3], gd_, sl, partials_);
