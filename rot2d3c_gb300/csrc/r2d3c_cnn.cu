@@ -49,6 +49,12 @@ constexpr int TH = 8, TW = 16, kThreads = 256;
 __device__ __forceinline__ unsigned pack_bf16(bf16 lo, bf16 hi) {
   return (unsigned)__bfloat16_as_ushort(lo) | ((unsigned)__bfloat16_as_ushort(hi) << 16);
 }
+// the gradient of a layer's result from that of its activation (rounded to
+// bf16) and GELU', two at a time
+__device__ __forceinline__ unsigned mul_bf16x2(unsigned da, float d0, float d1) {
+  return pack_bf16(__float2bfloat16_rn(__uint_as_float(da << 16) * d0),
+                   __float2bfloat16_rn(__uint_as_float(da & 0xFFFF0000u) * d1));
+}
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], const unsigned (&b)[2]) {
   asm volatile(
@@ -64,6 +70,17 @@ __device__ __forceinline__ float gelu_d(float x) {
   const float pdf = 0.39894228040143268f * __expf(-0.5f * x * x);
   return cdf + x * pdf;
 }
+
+// GELU(x), and its derivative in d
+__device__ __forceinline__ float gelu_both(float x, float& d) {
+  const float e = 1.0f + erff(x * 0.70710678118654752f);
+  const float pdf = 0.39894228040143268f * __expf(-0.5f * x * x);
+  d = 0.5f * e + x * pdf;
+  return 0.5f * x * e;
+}
+// the gradient of a layer's result from that of its activation (rounded to
+// bf16) and GELU'
+__device__ __forceinline__ bf16 mul_bf16(bf16 da, float d) { return __float2bfloat16_rn(__bfloat162float(da) * d); }
 
 // ---------------------------------------------------------------------------
 // Shared-memory tiles hold rows of C bf16 values (a pixel's channels, or a
@@ -110,7 +127,9 @@ __device__ __forceinline__ void stage_halo(bf16* s_in, const bf16* __restrict__ 
   constexpr int VPP = CIN / 8;
   for (int i = threadIdx.x; i < (TH + 2) * (TW + 2) * VPP; i += kThreads) {
     const int v = i % VPP, q = i / VPP, px = q % (TW + 2), py = q / (TW + 2);
-    const int gy = (ty0 + py - 1 + H) % H, gx = (tx0 + px - 1 + W) % W;
+    int gy = ty0 + py - 1, gx = tx0 + px - 1;
+    gy += gy < 0 ? H : (gy >= H ? -H : 0);
+    gx += gx < 0 ? W : (gx >= W ? -W : 0);
     *reinterpret_cast<uint4*>(s_in + tile_off<CIN>(q, v)) =
         reinterpret_cast<const uint4*>(in + (((size_t)b * H + gy) * W + gx) * CIN)[v];
   }
@@ -119,8 +138,11 @@ __device__ __forceinline__ void stage_halo(bf16* s_in, const bf16* __restrict__ 
 // ---------------------------------------------------------------------------
 // out[p][co] = sum_k in_col[p][k] w[k][co] (+ bias), periodic 3x3 stencil.
 // in: [B][H][W][CIN] bf16; w: [9*CIN][COUT] bf16; y: [B][H][W][cout_store] f32
-// (pre-activation, may be null); a: [B][H][W][COUT] bf16 = act(y) (may be
-// null); act: 0 identity, 1 GELU.  Requires H % TH == 0, W % TW == 0.
+// (may be null): the result, or with act the derivative GELU'(result), which
+// is all that the backward pass needs of it; a: [B][H][W][COUT] bf16 =
+// act(result), times mul where mul is set (the GELU' of the layer below, in the
+// backward pass; may be null); act: 0 identity, 1 GELU.  Requires H % TH == 0,
+// W % TW == 0.
 // Persistent CTAs: the weights are staged once, then the CTA loops over
 // 8 x 16 pixel tiles; warp w computes tile row w (16 pixels x COUT).
 // Fragments come from ldmatrix: A (pixels x k) directly, B (k x co) through
@@ -129,7 +151,8 @@ __device__ __forceinline__ void stage_halo(bf16* s_in, const bf16* __restrict__ 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kThreads)
 k_conv(const bf16* __restrict__ in, const bf16* __restrict__ w, const float* __restrict__ bias, int H, int W,
-       int ntiles, float* __restrict__ y, bf16* __restrict__ a, int act, int cout_store) {
+       int ntiles, float* __restrict__ y, bf16* __restrict__ a, int act, int cout_store,
+       const float* __restrict__ mul) {
   constexpr int NTN = COUT / 8;  // n-tiles
   static_assert(NTN % 2 == 0, "n-tiles in pairs");
   __shared__ __align__(128) bf16 s_in[(TH + 2) * (TW + 2) * CIN];
@@ -188,10 +211,18 @@ k_conv(const bf16* __restrict__ in, const bf16* __restrict__ w, const float* __r
         if (co >= cout_store) continue;
         const float v0 = acc[n][half * 2] + (bias ? bias[co] : 0.f);
         const float v1 = acc[n][half * 2 + 1] + (bias ? bias[co + 1] : 0.f);
-        if (y) *reinterpret_cast<float2*>(y + pix * cout_store + co) = make_float2(v0, v1);
-        if (a)
-          *reinterpret_cast<__nv_bfloat162*>(a + pix * COUT + co) =
-              __halves2bfloat162(__float2bfloat16_rn(act ? gelu(v0) : v0), __float2bfloat16_rn(act ? gelu(v1) : v1));
+        if (y)
+          *reinterpret_cast<float2*>(y + pix * cout_store + co) =
+              act ? make_float2(gelu_d(v0), gelu_d(v1)) : make_float2(v0, v1);
+        if (a) {
+          bf16 h0 = __float2bfloat16_rn(act ? gelu(v0) : v0), h1 = __float2bfloat16_rn(act ? gelu(v1) : v1);
+          if (mul) {
+            const float2 m = *reinterpret_cast<const float2*>(mul + pix * COUT + co);
+            h0 = mul_bf16(h0, m.x);
+            h1 = mul_bf16(h1, m.y);
+          }
+          *reinterpret_cast<__nv_bfloat162*>(a + pix * COUT + co) = __halves2bfloat162(h0, h1);
+        }
       }
     }
   }
@@ -296,41 +327,54 @@ struct TcConv {
   static constexpr int Y_UNITS = kTcPix * COUT / 4, A_UNITS = kTcPix * COUT / 8;
   static constexpr bool STAGE_IN_HALO = Y_UNITS + A_UNITS <= HALO_UNITS;
   static constexpr int STAGE_UNITS = STAGE_IN_HALO ? 0 : Y_UNITS + A_UNITS;
-  // two halo buffers (the next tile's is copied while this one's runs), the
-  // weights, the output staging, the mbarrier, the TMEM address and the bias
-  static constexpr size_t SMEM = (size_t)(2 * HALO_UNITS + W_UNITS + STAGE_UNITS) * 16 + 16 + 4 * 32;
+  // One halo buffer: five CTAs of 32 channels to an SM cover each other's copies
+  // better than three with a second buffer for the next tile's (a training step
+  // at 256^2, batch 32: 3.04 against 3.23 ms, an LES step of one image the same).
+  // Behind it the weights, the output staging, the mbarrier, the TMEM address and
+  // the bias.
+  static constexpr size_t SMEM = (size_t)(HALO_UNITS + W_UNITS + STAGE_UNITS) * 16 + 16 + 4 * 32;
 };
 
-// halo of tile t into buffer dst (one cp.async commit group; empty when
-// t >= ntiles)
+// halo of tile t into buffer dst (one cp.async commit group)
 template <int CIN>
-__device__ __forceinline__ void tc_stage_halo(uint4* dst, const bf16* __restrict__ in, int t, int ntiles, int H,
-                                              int W) {
+__device__ __forceinline__ void tc_stage_halo(uint4* dst, const bf16* __restrict__ in, int t, int H, int W) {
   constexpr int NCH = CIN / 8, HP = kTcPix + 2;
-  if (t < ntiles) {
-    const int tiles_x = W / kTcPix;
-    const int b = t / (tiles_x * H), gy = (t / tiles_x) % H, x0 = (t % tiles_x) * kTcPix;
-    for (int i = threadIdx.x; i < 3 * NCH * HP; i += kTcThreads) {
-      const int c = i % NCH, p = (i / NCH) % HP, r = i / (NCH * HP);
-      int sy = gy + r - 1, sx = x0 + p - 1;
-      sy += sy < 0 ? H : (sy >= H ? -H : 0);
-      sx += sx < 0 ? W : (sx >= W ? -W : 0);
-      tc_cp16(dst + (r * NCH + c) * HP + p, in + (((size_t)b * H + sy) * W + sx) * CIN + c * 8);
-    }
+  const int tiles_x = W / kTcPix;
+  const int b = t / (tiles_x * H), gy = (t / tiles_x) % H, x0 = (t % tiles_x) * kTcPix;
+  for (int i = threadIdx.x; i < 3 * NCH * HP; i += kTcThreads) {
+    const int c = i % NCH, p = (i / NCH) % HP, r = i / (NCH * HP);
+    int sy = gy + r - 1, sx = x0 + p - 1;
+    sy += sy < 0 ? H : (sy >= H ? -H : 0);
+    sx += sx < 0 ? W : (sx >= W ? -W : 0);
+    tc_cp16(dst + (r * NCH + c) * HP + p, in + (((size_t)b * H + sy) * W + sx) * CIN + c * 8);
   }
   tc_commit();
 }
 
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(kTcThreads)
+// What a launch writes besides the convolution: kPlain (inference, the gradient
+// of the input), kTrain (a hidden layer in training: GELU and GELU'), kBack (the
+// result times the GELU' of the layer below).  Separate instantiations, each
+// held to the registers that let its CTAs share an SM (shared memory: five, seven
+// at 16 output channels): with all three in one kernel, or without the bound (96
+// to 140 registers), a 256^2 LES step was 1.5-4% slower.
+//   The 32-channel layers at 256^2, batch 32: kTrain 193 us, bound by the issue of
+// erf and exp (57% of the slots); kBack 187, by the latency of its loads.  With
+// GELU' stored by the forward pass instead of recomputed from the pre-activation
+// by a pass of its own, that product folded in here, and the weight gradients'
+// copies under their products, a training step went 5.02 -> 3.04 ms.
+enum ConvMode { kPlain, kTrain, kBack };
+
+template <int CIN, int COUT, int MODE>
+__global__ void __launch_bounds__(kTcThreads, MODE == kPlain ? 7 : 5)
 k_conv_tc(const bf16* __restrict__ in, const bf16* __restrict__ wt, const float* __restrict__ bias, int H, int W,
-          int ntiles, float* __restrict__ y, bf16* __restrict__ a, int act, int cout_store, int* __restrict__ err) {
+          int ntiles, float* __restrict__ y, bf16* __restrict__ a, int act, int cout_store,
+          const float* __restrict__ mul, int* __restrict__ err) {
   using TC = TcConv<CIN, COUT>;
   constexpr int NCH = TC::NCH, HP = kTcPix + 2;
   constexpr unsigned IDESC = umma_idesc_bf16(kTcPix, COUT);
   extern __shared__ __align__(128) unsigned char tc_smem[];
-  uint4* s_halo = reinterpret_cast<uint4*>(tc_smem);  // two buffers
-  uint4* s_w = s_halo + 2 * TC::HALO_UNITS;
+  uint4* cur = reinterpret_cast<uint4*>(tc_smem);  // the tile's halo
+  uint4* s_w = cur + TC::HALO_UNITS;
   uint4* s_stage = s_w + TC::W_UNITS;  // own staging region (STAGE_UNITS)
   unsigned long long* s_bar = reinterpret_cast<unsigned long long*>(s_stage + TC::STAGE_UNITS);
   unsigned* s_tmem = reinterpret_cast<unsigned*>(s_bar + 1);
@@ -364,15 +408,24 @@ k_conv_tc(const bf16* __restrict__ in, const bf16* __restrict__ wt, const float*
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const unsigned tmem = *s_tmem;
   asm volatile("griddepcontrol.wait;\n" ::: "memory");  // the input activations are complete
-  tc_stage_halo<CIN>(s_halo, in, t, ntiles, H, W);
   const int tiles_x = W / kTcPix;
   unsigned phase = 0;
-  for (int it = 0; t < ntiles; t += gridDim.x, ++it) {
-    uint4* cur = s_halo + (it & 1) * TC::HALO_UNITS;
-    // the next tile's halo into the other buffer (its last reader, the
-    // previous tile's MMAs, has completed)
-    tc_stage_halo<CIN>(s_halo + ((it + 1) & 1) * TC::HALO_UNITS, in, t + gridDim.x, ntiles, H, W);
-    tc_wait<1>();  // weights and this tile's halo landed
+  for (; t < ntiles; t += gridDim.x) {
+    tc_stage_halo<CIN>(cur, in, t, H, W);
+    const int b = t / (tiles_x * H), gy = (t / tiles_x) % H, x0 = (t % tiles_x) * kTcPix;
+    const size_t pix0 = ((size_t)b * H + gy) * W + x0;  // the tile's pixels are contiguous
+    // GELU' of this thread's chunks of the copy-out, on its way with the halo
+    constexpr int NQ = MODE == kBack ? TC::A_UNITS / kTcThreads : 1;
+    float4 mm[NQ][2];
+    if constexpr (MODE == kBack) {
+      const float4* mp = reinterpret_cast<const float4*>(mul + pix0 * COUT);
+#pragma unroll
+      for (int j = 0; j < NQ; ++j) {
+        mm[j][0] = __ldcs(mp + 2 * (tid + j * kTcThreads));
+        mm[j][1] = __ldcs(mp + 2 * (tid + j * kTcThreads) + 1);
+      }
+    }
+    tc_wait<0>();  // weights and halo landed
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // visible to the tensor cores
     __syncthreads();
     if (tid == 0) {
@@ -412,41 +465,48 @@ k_conv_tc(const bf16* __restrict__ in, const bf16* __restrict__ wt, const float*
     // epilogue: pixel m = 32*warp + lane of the tile, COUT accumulators
     uint4* s_y = TC::STAGE_IN_HALO ? cur : s_stage;
     uint4* s_a = s_y + TC::Y_UNITS;
-    const int b = t / (tiles_x * H), gy = (t / tiles_x) % H, x0 = (t % tiles_x) * kTcPix;
-    const size_t pix0 = ((size_t)b * H + gy) * W + x0;  // the tile's pixels are contiguous
     const int m = warp * 32 + lane;
+    constexpr int YC = COUT / 4, AC = COUT / 8;  // 16-byte chunks per pixel row
     float v[COUT];
 #pragma unroll
     for (int co = 0; co < COUT; ++co) v[co] = __uint_as_float(r[co]) + s_bias[co];
-    if (y && cout_store < COUT) {
-      // the network output (2 channels): 8 bytes per pixel straight from registers
-#pragma unroll
-      for (int co = 0; co < COUT; co += 2)
-        if (co < cout_store) *reinterpret_cast<float2*>(y + (pix0 + m) * cout_store + co) = make_float2(v[co], v[co + 1]);
-    }
     // full rows go through the swizzled staging so that the global stores of
     // the tile are contiguous 16-byte chunks
-    constexpr int YC = COUT / 4, AC = COUT / 8;  // 16-byte chunks per pixel row
-    if (y && cout_store == COUT) {
+    auto stage_y = [&] {
 #pragma unroll
       for (int c = 0; c < YC; ++c)
         s_y[m * YC + (c ^ (m % YC))] = make_uint4(__float_as_uint(v[4 * c]), __float_as_uint(v[4 * c + 1]),
                                                   __float_as_uint(v[4 * c + 2]), __float_as_uint(v[4 * c + 3]));
-    }
+    };
+    if (MODE == kPlain && y && cout_store == COUT) stage_y();
     if (a) {
 #pragma unroll
       for (int c = 0; c < AC; ++c) {
         unsigned u[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float p0 = v[8 * c + 2 * e], p1 = v[8 * c + 2 * e + 1];
-          u[e] = pack_bf16(__float2bfloat16_rn(act ? gelu(p0) : p0), __float2bfloat16_rn(act ? gelu(p1) : p1));
+          float p0 = v[8 * c + 2 * e], p1 = v[8 * c + 2 * e + 1];
+          if constexpr (MODE == kTrain) {
+            p0 = gelu_both(p0, v[8 * c + 2 * e]);
+            p1 = gelu_both(p1, v[8 * c + 2 * e + 1]);
+          } else if (MODE == kPlain && act) {
+            p0 = gelu(p0);
+            p1 = gelu(p1);
+          }
+          u[e] = pack_bf16(__float2bfloat16_rn(p0), __float2bfloat16_rn(p1));
         }
         s_a[m * AC + (c ^ ((m / (8 / AC)) % AC))] = make_uint4(u[0], u[1], u[2], u[3]);
       }
     }
+    if (MODE == kPlain && y && cout_store < COUT) {
+      // the network output (2 channels): 8 bytes per pixel straight from registers
+#pragma unroll
+      for (int co = 0; co < COUT; co += 2)
+        if (co < cout_store) *reinterpret_cast<float2*>(y + (pix0 + m) * cout_store + co) = make_float2(v[co], v[co + 1]);
+    }
+    if (MODE == kTrain && cout_store == COUT) stage_y();  // (v holds GELU' by now)
     __syncthreads();  // staging complete; TMEM read before the next tile's MMAs
-    if (y && cout_store == COUT) {
+    if (MODE != kBack && y && cout_store == COUT) {
       uint4* gy4 = reinterpret_cast<uint4*>(y + pix0 * COUT);
       for (int q = tid; q < TC::Y_UNITS; q += kTcThreads) {
         const int mm = q / YC, c = q % YC;
@@ -455,14 +515,21 @@ k_conv_tc(const bf16* __restrict__ in, const bf16* __restrict__ wt, const float*
     }
     if (a) {
       uint4* ga4 = reinterpret_cast<uint4*>(a + pix0 * COUT);
-      for (int q = tid; q < TC::A_UNITS; q += kTcThreads) {
-        const int mm = q / AC, c = q % AC;
-        ga4[q] = s_a[mm * AC + (c ^ ((mm / (8 / AC)) % AC))];
+#pragma unroll
+      for (int j = 0; j < TC::A_UNITS / kTcThreads; ++j) {
+        const int q = tid + j * kTcThreads, px = q / AC, c = q % AC;
+        uint4 u = s_a[px * AC + (c ^ ((px / (8 / AC)) % AC))];
+        if constexpr (MODE == kBack) {
+          u.x = mul_bf16x2(u.x, mm[j][0].x, mm[j][0].y);
+          u.y = mul_bf16x2(u.y, mm[j][0].z, mm[j][0].w);
+          u.z = mul_bf16x2(u.z, mm[j][1].x, mm[j][1].y);
+          u.w = mul_bf16x2(u.w, mm[j][1].z, mm[j][1].w);
+        }
+        ga4[q] = u;
       }
     }
-    // the staging (possibly this tile's halo buffer, which the copy issued
-    // at the top of the next-but-one iteration refills) is free only after
-    // every thread's copy-out
+    // the staging (possibly the halo buffer, which the next iteration refills)
+    // is free only after every thread's copy-out
     if constexpr (TC::STAGE_IN_HALO) __syncthreads();
   }
   tc_wait<0>();  // no copy outlives the CTA
@@ -481,6 +548,31 @@ k_conv_tc(const bf16* __restrict__ in, const bf16* __restrict__ wt, const float*
 // warp w owns the m-tiles (16 rows of k) w, w+8, w+16 and all n-tiles.
 // Both fragments come from the transposing ldmatrix.
 // ---------------------------------------------------------------------------
+// The next tile's halo and gradient are copied (cp.async) into a second
+// buffer while the current tile's products run.
+template <int CIN, int COUT>
+__device__ __forceinline__ void wgrad_stage(bf16* s_in, bf16* s_dy, const bf16* __restrict__ in,
+                                            const bf16* __restrict__ dy, int t, int ntiles, int H, int W) {
+  if (t < ntiles) {
+    const int tiles_x = W / TW, tiles_y = H / TH;
+    const int b = t / (tiles_x * tiles_y);
+    const int ty0 = ((t / tiles_x) % tiles_y) * TH, tx0 = (t % tiles_x) * TW;
+    constexpr int VPP = CIN / 8, VPO = COUT / 8;
+    for (int i = threadIdx.x; i < (TH + 2) * (TW + 2) * VPP; i += kThreads) {
+      const int v = i % VPP, q = i / VPP, px = q % (TW + 2), py = q / (TW + 2);
+      int gy = ty0 + py - 1, gx = tx0 + px - 1;
+      gy += gy < 0 ? H : (gy >= H ? -H : 0);
+      gx += gx < 0 ? W : (gx >= W ? -W : 0);
+      tc_cp16(s_in + tile_off<CIN>(q, v), in + (((size_t)b * H + gy) * W + gx) * CIN + v * 8);
+    }
+    for (int i = threadIdx.x; i < TH * TW * VPO; i += kThreads) {
+      const int v = i % VPO, p = i / VPO, px = p % TW, py = p / TW;
+      tc_cp16(s_dy + tile_off<COUT>(p, v), dy + (((size_t)b * H + ty0 + py) * W + tx0 + px) * COUT + v * 8);
+    }
+  }
+  tc_commit();
+}
+
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kThreads)
 k_conv_wgrad(const bf16* __restrict__ in, const bf16* __restrict__ dy, int H, int W, int ntiles,
@@ -488,8 +580,8 @@ k_conv_wgrad(const bf16* __restrict__ in, const bf16* __restrict__ dy, int H, in
   constexpr int K = 9 * CIN, MT = K / 16, NTN = COUT / 8;
   constexpr int MPW = (MT + 7) / 8;  // m-tiles per warp (at most)
   static_assert(NTN % 2 == 0, "n-tiles in pairs");
-  __shared__ __align__(128) bf16 s_in[(TH + 2) * (TW + 2) * CIN];
-  __shared__ __align__(128) bf16 s_dy[TH * TW * COUT];
+  __shared__ __align__(128) bf16 s_in2[2][(TH + 2) * (TW + 2) * CIN];
+  __shared__ __align__(128) bf16 s_dy2[2][TH * TW * COUT];
   __shared__ float s_b[kThreads];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lj = lane >> 3, lr = lane & 7;
@@ -501,19 +593,15 @@ k_conv_wgrad(const bf16* __restrict__ in, const bf16* __restrict__ dy, int H, in
 #pragma unroll
       for (int r = 0; r < 4; ++r) acc[i][n][r] = 0.f;
   float bsum = 0.f;  // bias partial of channel threadIdx.x % COUT
-  const int tiles_x = W / TW, tiles_y = H / TH;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int b = t / (tiles_x * tiles_y);
-    const int ty0 = ((t / tiles_x) % tiles_y) * TH, tx0 = (t % tiles_x) * TW;
+  wgrad_stage<CIN, COUT>(s_in2[0], s_dy2[0], in, dy, blockIdx.x, ntiles, H, W);
+  int buf = 0;
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x, buf ^= 1) {
+    // (the other buffer's readers passed the barrier at the end of their tile)
+    wgrad_stage<CIN, COUT>(s_in2[buf ^ 1], s_dy2[buf ^ 1], in, dy, t + gridDim.x, ntiles, H, W);
+    tc_wait<1>();
     __syncthreads();
-    stage_halo<CIN>(s_in, in, b, ty0, tx0, H, W);
-    constexpr int VPO = COUT / 8;
-    for (int i = threadIdx.x; i < TH * TW * VPO; i += kThreads) {
-      const int v = i % VPO, p = i / VPO, px = p % TW, py = p / TW;
-      *reinterpret_cast<uint4*>(s_dy + tile_off<COUT>(p, v)) =
-          reinterpret_cast<const uint4*>(dy + (((size_t)b * H + ty0 + py) * W + tx0 + px) * COUT)[v];
-    }
-    __syncthreads();
+    const bf16* s_in = s_in2[buf];
+    const bf16* s_dy = s_dy2[buf];
     {  // bias: fixed pixel order per thread
       const int co = threadIdx.x % COUT;
       for (int p = threadIdx.x / COUT; p < TH * TW; p += kThreads / COUT)
@@ -544,7 +632,9 @@ k_conv_wgrad(const bf16* __restrict__ in, const bf16* __restrict__ dy, int H, in
         }
       }
     }
+    __syncthreads();
   }
+  tc_wait<0>();  // no copy outlives the CTA
   float* out = part + (size_t)blockIdx.x * (K * COUT + COUT);
   const int gid = lane >> 2, tig = lane & 3;
 #pragma unroll
@@ -572,15 +662,10 @@ __global__ void k_reduce_parts(const float* __restrict__ part, int nparts, int c
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   float s = 0.f;
+  // (38 loads in flight together, 64-thread blocks: 21 -> 17 us for the 304 partials)
+#pragma unroll 38
   for (int c = 0; c < nparts; ++c) s += part[(size_t)c * count + i];
   grad[i] = s;
-}
-
-// dY' = dA * gelu'(y) (bf16), for the hidden layers
-__global__ void k_gelu_back(const bf16* __restrict__ da, const float* __restrict__ y, size_t count,
-                            bf16* __restrict__ dy) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
-    dy[i] = __float2bfloat16_rn(__bfloat162float(da[i]) * gelu_d(y[i]));
 }
 
 // MSE loss of the 2 output channels against the target; dY of the last
@@ -591,16 +676,13 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
   __shared__ float red[256];
   float s = 0.f;
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x) {
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      float g = 0.f;
-      if (c < 2) {
-        const float d = out[p * 2 + c] - (tgt[p * 2 + c] - tmean[c]) / tsd[c];
-        s += d * d;
-        g = 2.f * d * scale;
-      }
-      dy[p * 16 + c] = __float2bfloat16_rn(g);
-    }
+    const float2 o = reinterpret_cast<const float2*>(out)[p];
+    const float d0 = o.x - (tgt[p * 2] - tmean[0]) / tsd[0], d1 = o.y - (tgt[p * 2 + 1] - tmean[1]) / tsd[1];
+    s += d0 * d0;
+    s += d1 * d1;
+    uint4* q = reinterpret_cast<uint4*>(dy + p * 16);
+    q[0] = make_uint4(pack_bf16(__float2bfloat16_rn(2.f * d0 * scale), __float2bfloat16_rn(2.f * d1 * scale)), 0, 0, 0);
+    q[1] = make_uint4(0, 0, 0, 0);
   }
   red[threadIdx.x] = s;
   __syncthreads();
@@ -682,14 +764,27 @@ __global__ void k_unpad_wgrad(const float* __restrict__ gp, int cin, int cout, i
   }
 }
 
-// FP32 NHWC [npix][c] -> bf16 NHWC [npix][cp], (x - mean[ch]) / std[ch],
-// zero padding channels
-__global__ void k_to_bf16(const float* __restrict__ x, size_t npix, int c, int cp, const float* __restrict__ mean,
+// the network's input: FP32 NHWC, 8 channels -> bf16 NHWC, 16 channels,
+// (x - mean[ch]) / std[ch], the padding channels zero; a pixel per thread in
+// 16-byte accesses
+__global__ void k_to_bf16(const float* __restrict__ x, size_t npix, const float* __restrict__ mean,
                           const float* __restrict__ sd, bf16* __restrict__ out) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < npix * cp; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t p = i / cp;
-    const int ch = (int)(i % cp);
-    out[i] = __float2bfloat16_rn(ch < c ? (x[p * c + ch] - mean[ch]) / sd[ch] : 0.f);
+  float m[8], d[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    m[c] = mean[c];
+    d[c] = sd[c];
+  }
+  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < npix; p += (size_t)gridDim.x * blockDim.x) {
+    float v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = (x[p * 8 + c] - m[c]) / d[c];
+    uint4* q = reinterpret_cast<uint4*>(out + p * 16);
+    unsigned u[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) u[e] = pack_bf16(__float2bfloat16_rn(v[2 * e]), __float2bfloat16_rn(v[2 * e + 1]));
+    q[0] = make_uint4(u[0], u[1], u[2], u[3]);
+    q[1] = make_uint4(0, 0, 0, 0);
   }
 }
 
@@ -723,14 +818,14 @@ int resident_ctas(K k) {
 
 template <int CIN, int COUT>
 void conv_launch(const bf16* in, const bf16* w, const float* b, int B, int H, int W, float* y, bf16* a, int act,
-                 int cout_store, int ctas, cudaStream_t st) {
+                 int cout_store, const float* mul, int ctas, cudaStream_t st) {
   const int tiles = B * (H / TH) * (W / TW);
-  k_conv<CIN, COUT><<<std::min(tiles, ctas), kThreads, 0, st>>>(in, w, b, H, W, tiles, y, a, act, cout_store);
+  k_conv<CIN, COUT><<<std::min(tiles, ctas), kThreads, 0, st>>>(in, w, b, H, W, tiles, y, a, act, cout_store, mul);
 }
 
-template <int CIN, int COUT>
-void conv_tc_launch(const bf16* in, const bf16* w, const float* b, int B, int H, int W, float* y, bf16* a, int act,
-                    int cout_store, int ctas, int* err, cudaStream_t st) {
+template <int CIN, int COUT, int MODE>
+void conv_tc_launch_as(const bf16* in, const bf16* w, const float* b, int B, int H, int W, float* y, bf16* a, int act,
+                    int cout_store, const float* mul, int ctas, int* err, cudaStream_t st) {
   const int tiles = B * H * (W / kTcPix);
   // programmatic stream serialisation: the prologue overlaps the preceding
   // kernel's tail (k_conv_tc waits before its first read of `in`)
@@ -744,23 +839,32 @@ void conv_tc_launch(const bf16* in, const bf16* w, const float* b, int B, int H,
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cuda_check(cudaLaunchKernelEx(&cfg, k_conv_tc<CIN, COUT>, in, w, b, H, W, tiles, y, a, act, cout_store, err),
+  cuda_check(cudaLaunchKernelEx(&cfg, k_conv_tc<CIN, COUT, MODE>, in, w, b, H, W, tiles, y, a, act, cout_store, mul,
+                                err),
              "k_conv_tc");
 }
 template <int CIN, int COUT>
-int resident_tc_ctas() {
-  cuda_check(cudaFuncSetAttribute(k_conv_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+void conv_tc_launch(const bf16* in, const bf16* w, const float* b, int B, int H, int W, float* y, bf16* a, int act,
+                    int cout_store, const float* mul, const int* ctas, int* err, cudaStream_t st) {
+  if (mul) conv_tc_launch_as<CIN, COUT, kBack>(in, w, b, B, H, W, y, a, act, cout_store, mul, ctas[kBack], err, st);
+  else if (act && y)
+    conv_tc_launch_as<CIN, COUT, kTrain>(in, w, b, B, H, W, y, a, act, cout_store, mul, ctas[kTrain], err, st);
+  else conv_tc_launch_as<CIN, COUT, kPlain>(in, w, b, B, H, W, y, a, act, cout_store, mul, ctas[kPlain], err, st);
+}
+template <int CIN, int COUT, int MODE>
+int resident_tc_ctas_as() {
+  cuda_check(cudaFuncSetAttribute(k_conv_tc<CIN, COUT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)TcConv<CIN, COUT>::SMEM),
              "cudaFuncSetAttribute(max dynamic smem)");
   // the whole unified L1/shared array as shared memory, so that several
   // CTAs (and their copy pipelines) share each SM
-  cuda_check(cudaFuncSetAttribute(k_conv_tc<CIN, COUT>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  cuda_check(cudaFuncSetAttribute(k_conv_tc<CIN, COUT, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                   (int)cudaSharedmemCarveoutMaxShared),
              "cudaFuncSetAttribute(carveout)");
   int dev = 0, sms = 0, per_sm = 0, smem_sm = 0, reserved = 0;
   cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
   cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
-  cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv_tc<CIN, COUT>, kTcThreads,
+  cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_conv_tc<CIN, COUT, MODE>, kTcThreads,
                                                            TcConv<CIN, COUT>::SMEM),
              "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
   // the shared-memory bound itself (with the carveout at its maximum)
@@ -769,6 +873,13 @@ int resident_tc_ctas() {
   cuda_check(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev), "cudaDeviceGetAttribute");
   const int by_smem = smem_sm / (int)(TcConv<CIN, COUT>::SMEM + reserved);
   return std::max(1, std::max(per_sm, std::min(by_smem, 8))) * sms;
+}
+
+template <int CIN, int COUT>
+void resident_tc_ctas(int (&ctas)[3]) {
+  ctas[kPlain] = resident_tc_ctas_as<CIN, COUT, kPlain>();
+  ctas[kTrain] = resident_tc_ctas_as<CIN, COUT, kTrain>();
+  ctas[kBack] = resident_tc_ctas_as<CIN, COUT, kBack>();
 }
 
 template <int CIN, int COUT>
@@ -783,7 +894,7 @@ struct r2d3c_cnn {
   int H = 0, W = 0, Bmax = 0;
   unsigned long long serial = 0;  // unique per network created in this process
   int ctas[3] = {};               // resident CTAs of k_conv<16,32>, <32,32>, <32,16>
-  int tc_ctas[3] = {};            // and of k_conv_tc
+  int tc_ctas[3][3] = {};         // and of k_conv_tc, by its mode
   bool use_tc = false;            // tcgen05 convolutions (W % 128 == 0)
   int* err = nullptr;             // set by a device wait that gave up
   cudaStream_t st = nullptr;
@@ -795,7 +906,7 @@ struct r2d3c_cnn {
   bf16* wtf[kLayers] = {};  // forward / backward-data weights in the UMMA layout
   bf16* wtb[kLayers] = {};
   bf16* act[kLayers + 1] = {};   // act[0] = bf16 input (16 ch), act[l+1] = layer l output (bf16)
-  float* pre[kLayers] = {};      // pre-activations y (f32), last = network output (2 ch)
+  float* pre[kLayers] = {};      // GELU' of the hidden layers (f32), last = network output (2 ch)
   bf16 *dA = nullptr, *dY = nullptr;
   float* part = nullptr;
   float* lpart = nullptr;
@@ -825,22 +936,24 @@ struct r2d3c_cnn {
       throw Error(kETIMEOUT, "a tensor-core convolution wait gave up");
     }
   }
-  void conv(int l, const bf16* in, const bf16* w, int B, float* y, bf16* a, int act_on, bool bias, bool back) {
+  // (mul: GELU' of the layer below, which the backward-data result is multiplied by)
+  void conv(int l, const bf16* in, const bf16* w, int B, float* y, bf16* a, int act_on, bool bias, bool back,
+            const float* mul = nullptr) {
     const float* b = bias ? wm + L[l].boff : nullptr;
     // forward shapes (CINP, COUTP) or backward-data shapes (COUTP, CINP)
     const int ci = back ? L[l].coutp : L[l].cinp, co = back ? L[l].cinp : L[l].coutp;
     const int store = back ? co : (l == kLayers - 1 ? L[l].cout : co);
     if (use_tc) {
       const bf16* wt = back ? wtb[l] : wtf[l];  // the same matrix as w, UMMA layout
-      if (ci == 16 && co == 32) conv_tc_launch<16, 32>(in, wt, b, B, H, W, y, a, act_on, store, tc_ctas[0], err, st);
+      if (ci == 16 && co == 32) conv_tc_launch<16, 32>(in, wt, b, B, H, W, y, a, act_on, store, mul, tc_ctas[0], err, st);
       else if (ci == 32 && co == 32)
-        conv_tc_launch<32, 32>(in, wt, b, B, H, W, y, a, act_on, store, tc_ctas[1], err, st);
+        conv_tc_launch<32, 32>(in, wt, b, B, H, W, y, a, act_on, store, mul, tc_ctas[1], err, st);
       else if (ci == 32 && co == 16)
-        conv_tc_launch<32, 16>(in, wt, b, B, H, W, y, a, act_on, store, tc_ctas[2], err, st);
+        conv_tc_launch<32, 16>(in, wt, b, B, H, W, y, a, act_on, store, mul, tc_ctas[2], err, st);
       else throw Error(kEINVAL, "unsupported conv shape");
-    } else if (ci == 16 && co == 32) conv_launch<16, 32>(in, w, b, B, H, W, y, a, act_on, store, ctas[0], st);
-    else if (ci == 32 && co == 32) conv_launch<32, 32>(in, w, b, B, H, W, y, a, act_on, store, ctas[1], st);
-    else if (ci == 32 && co == 16) conv_launch<32, 16>(in, w, b, B, H, W, y, a, act_on, store, ctas[2], st);
+    } else if (ci == 16 && co == 32) conv_launch<16, 32>(in, w, b, B, H, W, y, a, act_on, store, mul, ctas[0], st);
+    else if (ci == 32 && co == 32) conv_launch<32, 32>(in, w, b, B, H, W, y, a, act_on, store, mul, ctas[1], st);
+    else if (ci == 32 && co == 16) conv_launch<32, 16>(in, w, b, B, H, W, y, a, act_on, store, mul, ctas[2], st);
     else throw Error(kEINVAL, "unsupported conv shape");
     cuda_check(cudaGetLastError(), "k_conv");
   }
@@ -854,11 +967,11 @@ struct r2d3c_cnn {
   }
 
   // forward of a batch of B inputs (f32 NHWC 8 ch) -> pre[kLayers-1] (f32 NHWC 2 ch);
-  // the hidden layers' pre-activations (kept for the backward pass) are
-  // written only when train is set
+  // the hidden layers' GELU' (kept for the backward pass) is written only when
+  // train is set
   void forward(const float* x, int B, bool train) {
     const size_t npix = (size_t)B * H * W;
-    k_to_bf16<<<1024, 256, 0, st>>>(x, npix, 8, 16, norm, norm + 8, act[0]);
+    k_to_bf16<<<1024, 256, 0, st>>>(x, npix, norm, norm + 8, act[0]);
     cuda_check(cudaGetLastError(), "k_to_bf16");
     layers(B, train);
   }
@@ -887,7 +1000,7 @@ struct r2d3c_cnn {
   }
 
   // From dY = dL/dy of the last layer (as the forward pass left it, with
-  // the hidden pre-activations kept): the parameter gradients into grad[]
+  // the hidden layers' GELU' kept): the parameter gradients into grad[]
   // and, when gx is set, dL/dx of the FP32 input into gx
   void backprop(int B, float* gx) {
     const size_t npix = (size_t)B * H * W;
@@ -897,7 +1010,7 @@ struct r2d3c_cnn {
       wgrad(l, act[l], dY, B);
       // per-CTA partials: 9*cinp*coutp weight entries, then coutp bias entries
       const int kc = 9 * ly.cinp * ly.coutp + ly.coutp;
-      k_reduce_parts<<<(kc + 255) / 256, 256, 0, st>>>(part, nparts, kc, part + (size_t)nparts * kc);
+      k_reduce_parts<<<(kc + 63) / 64, 64, 0, st>>>(part, nparts, kc, part + (size_t)nparts * kc);
       cuda_check(cudaGetLastError(), "k_reduce_parts");
       // unpad into grad (layout [9][cin][cout], then the bias)
       unpad_wgrad(l, part + (size_t)nparts * kc);
@@ -910,10 +1023,9 @@ struct r2d3c_cnn {
         }
         break;
       }
-      // then dY' = dA * gelu'(pre[l-1])
-      conv(l, dY, wb[l], B, nullptr, dA, 0, false, true);
-      k_gelu_back<<<1024, 256, 0, st>>>(dA, pre[l - 1], npix * L[l - 1].coutp, dY);
-      cuda_check(cudaGetLastError(), "k_gelu_back");
+      // and dY' = dA * gelu'(layer l - 1), which pre[l - 1] holds, in one pass
+      conv(l, dY, wb[l], B, nullptr, dA, 0, false, true, pre[l - 1]);
+      std::swap(dA, dY);
     }
   }
 
@@ -1024,9 +1136,9 @@ int r2d3c_cnn_create(int H, int W, int max_batch, int seed, r2d3c_cnn** out) {
       throw Error(kEINVAL, "R2D3C_CNN_CONV must be mma or tcgen05");
     c->use_tc = W % kTcPix == 0 && !(conv_env && std::strcmp(conv_env, "mma") == 0);
     if (c->use_tc) {
-      c->tc_ctas[0] = resident_tc_ctas<16, 32>();
-      c->tc_ctas[1] = resident_tc_ctas<32, 32>();
-      c->tc_ctas[2] = resident_tc_ctas<32, 16>();
+      resident_tc_ctas<16, 32>(c->tc_ctas[0]);
+      resident_tc_ctas<32, 32>(c->tc_ctas[1]);
+      resident_tc_ctas<32, 16>(c->tc_ctas[2]);
     }
     cuda_check(cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking), "cudaStreamCreate");
     size_t off = 0;
