@@ -1244,12 +1244,13 @@ class EngineT final : public IEngine {
         }
         if (fuse && !kFuseCA<T, N>) throw Error(kESTATE, "pass C carries pass A only for FP32 n <= 512");
         const int groups = (gd_.M + NT - 1) / NT;
-        const int g = gc_ ? gc_ : C::G;  // groups per CTA: autotuned
+        const int gc = fuse ? gf_ : gc_;
+        const int g = gc ? gc : C::G;  // groups per CTA: autotuned
         // the C1 and C2 updates of a column pair in one CTA or two, and
         // teams of wc_ groups per column pair (autotuned)
-        const int w = kChunkC<T, N> ? wc_ : 1;
+        const int w = kChunkC<T, N> ? (fuse ? wf_ : wc_) : 1;
         const int teams = std::max(1, g / w);
-        const dim3 grid((groups + teams - 1) / teams, nb, kChunkC<T, N> ? fc_ : 1);
+        const dim3 grid((groups + teams - 1) / teams, nb, kChunkC<T, N> ? (fuse ? ff_ : fc_) : 1);
         k<<<grid, C::TPF * g, g * PassSmem<T, N>::GROUP_ELEMS * sizeof(cpx<T>), st_>>>(pb_, c1in, c2in, pbase_[P_PS], pbase_[P_VZ],
                                                            pbase_[P_FP], pbase_[P_FZ], c1out, c2out, gd_, d_sc_,
                                                            scal_base_, o, tw_, batch(), t5, t6, w,
@@ -1513,9 +1514,24 @@ class EngineT final : public IEngine {
           wc_ = cands[i].wide;
           launch_passC(c1, c2, c3, c4, 4, nb_);
         });
+        // with the next substep's pass A in it (fuse_ca()) pass C has its own
+        // fastest shape: in the one that is fastest without, a 256^2 step took
+        // 55.5 us instead of 49.3 in a third of the contexts
+        std::vector<float> us_f;
+        if (kFuseCA<T, N> && nb_ == 1) {
+          passc_mode_ = 0;
+          us_f = time_candidates(cands.size(), [&](size_t i) {
+            if (cands[i].mode) return;
+            gf_ = cands[i].grid;
+            ff_ = cands[i].chunks;
+            wf_ = cands[i].wide;
+            launch_passC(c1, c2, c3, c4, 4, nb_, true);
+          });
+        }
         tune_c_.clear();
         for (size_t i = 0; i < cands.size(); ++i) {
           TuneRec r{cands[i].mode, cands[i].grid, us[i]};
+          if (!us_f.empty()) r.us_fused = us_f[i];
           r.chunks = cands[i].chunks;
           r.wide = cands[i].wide;
           tune_c_.push_back(r);
@@ -1634,6 +1650,19 @@ class EngineT final : public IEngine {
       // a forced pass-C group count without a forced team width runs one group per column pair
       wc_ = forced[5] > 0 ? forced[5] : forced[3] >= 0 ? 1 : (c0 < tune_c_.size() ? tune_c_[c0].wide : 1);
       if (!kChunkC<T, N>) fc_ = wc_ = 1;
+      gf_ = gc_;
+      ff_ = fc_;
+      wf_ = wc_;
+      if (forced[3] < 0 && forced[4] < 0 && forced[5] < 0) {
+        float best = 0.f;
+        for (const TuneRec& t : tune_c_)
+          if (t.mode == 0 && t.us_fused > 0.f && (best == 0.f || t.us_fused < best)) {
+            best = t.us_fused;
+            gf_ = t.grid;
+            ff_ = t.chunks;
+            wf_ = t.wide;
+          }
+      }
       if (wc_ > gc_) throw Error(kEINVAL, "R2D3C_GROUPS: pass C team wider than its groups per CTA");
     });
   }
@@ -1731,6 +1760,7 @@ class EngineT final : public IEngine {
   int ga_ = 0, fa_ = 1;  // pass A: groups per CTA (0: the config's G), field chunks (autotuned)
   int fc_ = 1;           // pass C: CTAs per column pair (1 or 2, autotuned)
   int wc_ = 1;           // pass C: groups per column pair sharing its update (autotuned)
+  int gf_ = 0, ff_ = 1, wf_ = 1;  // the same of pass C with the next substep's pass A
   int gb_ = 0, gc_ = 0;  // passes B, C one CTA per row / column pair: groups per CTA (autotuned)
   struct TuneRec {
     int mode, grid;  // pass A: groups, field chunks; B, C: variant, CTAs or groups
@@ -1738,6 +1768,7 @@ class EngineT final : public IEngine {
     int radix = 0;   // pass A: the transform radix
     int chunks = 1;  // pass C: CTAs per column pair
     int wide = 1;    // pass C: groups per column pair
+    float us_fused = 0.f;  // pass C with the next substep's pass A
   };
   // pass A radix chosen per (precision, n), shared by the engines of a process
   static std::map<int, int>& radix_cache() {
