@@ -66,8 +66,8 @@ struct Cfg {
 // Transforms carried at once by one group in passes A, B and C.  Two in the
 // FP32 path: pass A and C transform two adjacent kx columns, pass B two
 // adjacent rows, and the mixed planes use the pair-tiled layout below so that
-// every access moves whole 32-byte sectors.  One in the FP64 path, which has
-// passes of its own (r2d3c_pass64.cuh).
+// every access moves whole 32-byte sectors.  One in the FP64 path, whose own
+// passes (r2d3c_pass64.cuh) carry one transform a group over the same layout.
 template <typename T, int N> struct PassNT {
   static constexpr int value = sizeof(T) == 4 ? 2 : 1;
 };
@@ -323,7 +323,7 @@ k_passA(const cpx<T>* __restrict__ ps, const cpx<T>* __restrict__ vz, cpx<T>* __
   for (int q = 0; q < C::E; ++q) kyi[q] = ky_of(lane + q * C::TPF, N);
   // The source column (pair) is re-read for every field, from L2, rather
   // than held in registers across the fields: the registers freed let FP32
-  // run two 256-thread CTAs per SM (and keep FP64 from spilling)
+  // run two 256-thread CTAs per SM
   cpx<T> v[NT][C::E];
   auto src_at = [&](const cpx<T>* sp, int t, int q) -> cpx<T> {
     const int col = kx0 + t, ky = kyi[q];
@@ -884,8 +884,7 @@ struct RkIn {
 // New C1 (rk_apply1) and C2 (rk_apply2) of one element
 // (Rot2D3C.para.f90:580-599); zero outside the retained disc and at k = 0.
 // Both components are divided by the same implicit divisor: one reciprocal
-// and two products (within an ulp of the two quotients; an FP64 division
-// is a long sequence on the FP64 pipe, which binds the FP64 path).
+// and two products (within an ulp of the two quotients).
 // The two are independent: C1 needs C2's input (the Coriolis term 2 Omega
 // d_y C2) and [psi, -k^2 psi], C2 needs C1's input and [psi, vz].
 template <typename T>

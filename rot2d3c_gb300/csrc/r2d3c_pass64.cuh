@@ -4,10 +4,10 @@
 // SM and clock) where integers can do it.
 //
 // Per launch at 4096^2 (us; FP64 arithmetic, the transforms alone in fixed
-// point, these kernels): A 2556, 841, 385; B 5227, 1697, 957; C 1179, 594,
-// 331.  What bounds them now (ncu): A and B the issue of integer instructions
-// (51-54% of the slots, ALU pipe 54%), C the FP64 pipe of the update (55%)
-// and the latency of its loads; DRAM 11-27% of peak.
+// point, these kernels): A 2556, 841, 381; B 5227, 1697, 942; C 1179, 594,
+// 270.  What bounds them now (ncu): A and B the issue of integer instructions
+// (50-55% of the slots, ALU pipe 54-55%), C the FP64 pipe of the update (70%)
+// and the latency of its loads; DRAM 11-33% of peak.
 #pragma once
 
 #include "r2d3c_kernels.cuh"
