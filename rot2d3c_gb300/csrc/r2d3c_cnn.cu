@@ -361,7 +361,7 @@ __device__ __forceinline__ void tc_stage_halo(uint4* dst, const bf16* __restrict
 // at 16 output channels): with all three in one kernel, or without the bound (96
 // to 140 registers), a 256^2 LES step was 1.5-4% slower.
 //   The 32-channel layers at 256^2, batch 32: kTrain 193 us, bound by the issue of
-// erf and exp (57% of the slots); kBack 187, by the latency of its loads.  With
+// erf and exp (57% of the slots); kBack 146, by the latency of its loads.  With
 // GELU' stored by the forward pass instead of recomputed from the pre-activation
 // by a pass of its own, that product folded in here, and the weight gradients'
 // copies under their products, a training step went 5.02 -> 3.04 ms.
@@ -844,15 +844,36 @@ k_conv_wgrad_tc(const bf16* __restrict__ in, const bf16* __restrict__ dy, int H,
   }
 }
 
-// grad[i] = sum_c part[c][i] in fixed order
-__global__ void k_reduce_parts(const float* __restrict__ part, int nparts, int count, float* __restrict__ grad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
+// Sums over the CTAs' partials (9*cinp*coutp weight entries, coutp bias entries
+// each), in fixed order, into the parameter layout: g[9][cin][cout], gb[cout].  A
+// block takes 32 entries and eight segments of the partials, 38 loads of a thread
+// in flight together.  Latency-bound; one thread per entry (38 loads in flight, then
+// the next 38, and a kernel of its own for the layout) took 17 + 3 us a layer at
+// 32 channels and 304 partials, this 6.
+constexpr int kRedSeg = 8;
+__global__ void __launch_bounds__(32 * kRedSeg)
+k_reduce_parts(const float* __restrict__ part, int nparts, int cin, int cout, int cinp, int coutp,
+               float* __restrict__ g, float* __restrict__ gb) {
+  __shared__ float red[kRedSeg][32];
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane, nw = 9 * cin * cout;
+  const size_t count = (size_t)9 * cinp * coutp + coutp;
   float s = 0.f;
-  // (38 loads in flight together, 64-thread blocks: 21 -> 17 us for the 304 partials)
+  if (i < nw + cout) {
+    const int co = i % cout, ci = (i / cout) % cin, tap = i / (cout * cin);
+    const float* p = part + (i < nw ? (tap * cinp + ci) * coutp + co : 9 * cinp * coutp + (i - nw));
+    const int per = (nparts + kRedSeg - 1) / kRedSeg, c1 = min(nparts, (seg + 1) * per);
 #pragma unroll 38
-  for (int c = 0; c < nparts; ++c) s += part[(size_t)c * count + i];
-  grad[i] = s;
+    for (int c = seg * per; c < c1; ++c) s += p[(size_t)c * count];
+  }
+  red[seg][lane] = s;
+  __syncthreads();
+  if (seg == 0 && i < nw + cout) {
+#pragma unroll
+    for (int k = 1; k < kRedSeg; ++k) s += red[k][lane];
+    if (i < nw) g[i] = s;
+    else gb[i - nw] = s;
+  }
 }
 
 // MSE loss of the 2 output channels against the target; dY of the last
@@ -935,20 +956,6 @@ __global__ void k_pack_weights(const float* __restrict__ wm, int cin, int cout, 
   wb[(size_t)kb * cinp + ci] = h;
   wtf[((size_t)(kf >> 3) * coutp + co) * 8 + (kf & 7)] = h;
   wtb[((size_t)(kb >> 3) * cinp + ci) * 8 + (kb & 7)] = h;
-}
-
-// padded weight gradient [9][cinp][coutp] -> parameter layout [9][cin][cout];
-// the padded bias gradient (coutp entries after the weights) -> gb[cout]
-__global__ void k_unpad_wgrad(const float* __restrict__ gp, int cin, int cout, int cinp, int coutp,
-                              float* __restrict__ g, float* __restrict__ gb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nw = 9 * cin * cout;
-  if (i < nw) {
-    const int co = i % cout, ci = (i / cout) % cin, tap = i / (cout * cin);
-    g[i] = gp[((size_t)tap * cinp + ci) * coutp + co];
-  } else if (i < nw + cout) {
-    gb[i - nw] = gp[(size_t)9 * cinp * coutp + (i - nw)];
-  }
 }
 
 // the network's input: FP32 NHWC, 8 channels -> bf16 NHWC, 16 channels,
@@ -1215,12 +1222,9 @@ struct r2d3c_cnn {
       const Layer& ly = L[l];
       // dY holds dL/dy of layer l (bf16, coutp channels)
       wgrad(l, act[l], dY, B);
-      // per-CTA partials: 9*cinp*coutp weight entries, then coutp bias entries
-      const int kc = 9 * ly.cinp * ly.coutp + ly.coutp;
-      k_reduce_parts<<<(kc + 63) / 64, 64, 0, st>>>(part, nparts, kc, part + (size_t)nparts * kc);
+      k_reduce_parts<<<(9 * ly.cin * ly.cout + ly.cout + 31) / 32, 32 * kRedSeg, 0, st>>>(
+          part, nparts, ly.cin, ly.cout, ly.cinp, ly.coutp, grad + ly.woff, grad + ly.boff);
       cuda_check(cudaGetLastError(), "k_reduce_parts");
-      // unpad into grad (layout [9][cin][cout], then the bias)
-      unpad_wgrad(l, part + (size_t)nparts * kc);
       // dA of layer l's input = conv(dY, wb[l]) (backward data)
       if (l == 0) {
         if (gx) {
@@ -1234,14 +1238,6 @@ struct r2d3c_cnn {
       conv(l, dY, wb[l], B, nullptr, dA, 0, false, true, pre[l - 1]);
       std::swap(dA, dY);
     }
-  }
-
-  void unpad_wgrad(int l, const float* gp) {
-    const Layer& ly = L[l];
-    const int c = 9 * ly.cin * ly.cout + ly.cout;
-    k_unpad_wgrad<<<(c + 255) / 256, 256, 0, st>>>(gp, ly.cin, ly.cout, ly.cinp, ly.coutp, grad + ly.woff,
-                                                    grad + ly.boff);
-    cuda_check(cudaGetLastError(), "k_unpad_wgrad");
   }
 
   void pack() {
@@ -1387,7 +1383,7 @@ int r2d3c_cnn_create(int H, int W, int max_batch, int seed, r2d3c_cnn** out) {
     for (int l = 0; l < kLayers; ++l) c->act[l + 1] = c->alloc<bf16>(npix * kCoutPad[l]);
     c->dA = c->alloc<bf16>(npix * 32);
     c->dY = c->alloc<bf16>(npix * 32);  // dL/dy of the current layer (<= 32 channels)
-    c->part = c->alloc<float>((size_t)(c->nparts + 1) * (9 * 32 * 32 + 32));
+    c->part = c->alloc<float>((size_t)c->nparts * (9 * 32 * 32 + 32));
     c->lpart = c->alloc<float>(256);
     c->norm = c->alloc<float>(20);
     c->err = c->alloc<int>(1);
