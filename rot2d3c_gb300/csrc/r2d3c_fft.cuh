@@ -133,6 +133,24 @@ __device__ __forceinline__ void fft_sync() {
   }
 }
 
+// Largest value of a transform group's TPF threads (of the warp's, above 32), in
+// all of them.  On small grids a block, or its last warp, has fewer than 32
+// threads: the lanes that do not exist count as exited (the full mask may name
+// them), but a value shuffled from one is undefined, so no offset leaves the group.
+template <int TPF>
+constexpr int kGroupLanes = TPF < 32 ? TPF : 32;
+template <int TPF, typename V>
+__device__ __forceinline__ V group_max(V v) {
+#pragma unroll
+  for (int o = kGroupLanes<TPF> / 2; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+// the thread that stands for the group (the warp) after group_max
+template <int TPF>
+__device__ __forceinline__ bool group_first() {
+  return (threadIdx.x & (kGroupLanes<TPF> - 1)) == 0;
+}
+
 // NT independent length-N transforms carried by the same TPF = N/E threads
 // (thread `lane` holds v[t][q] = x_t[lane + q*TPF]).  The NT transforms share
 // every twiddle load and every barrier.  Shared memory: NT interleaved

@@ -239,12 +239,9 @@ k_rowc2r(const cpx<T>* __restrict__ tin, T* __restrict__ rout,
       mx = fmax(mx, fmax((double)v[0][q].x, (double)v[0][q].y));
       mn = fmin(mn, fmin((double)v[0][q].x, (double)v[0][q].y));
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      mn = fmin(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
+    mx = group_max<C::TPF>(mx);
+    mn = -group_max<C::TPF>(-mn);
+    if (group_first<C::TPF>()) {
       atomicMax(&mm_enc[0], enc_ordered(mx));
       atomicMax(&mm_enc[1], enc_ordered(-mn));
     }
@@ -436,19 +433,19 @@ __device__ __forceinline__ void packed_pair(const cpx<T>* __restrict__ pa, const
 // --------------------------------------------------------------------------
 // CFL maximum of |grad psi|^2 = x^2 + y^2 over a thread's values of
 // z1 = d_x psi + i d_y psi (CFL_condition, pseudospec2D_Rot2D3C.f90:867-874),
-// folded into the run's encoded maximum.  The squares are formed in the
+// folded into the run's encoded maximum (`on`: for this group's; every thread of
+// the warp calls it).  The squares are formed in the
 // compute type (an FP64 square per value would double the FP32 pass's time
 // on GB300's FP64 rate); the maximum is kept in FP64.
-template <typename T, int NT, int E>
-__device__ __forceinline__ void cfl_max_sq(const cpx<T> (&v)[NT][E], unsigned long long* enc) {
+template <typename T, int NT, int E, int TPF>
+__device__ __forceinline__ void cfl_max_sq(const cpx<T> (&v)[NT][E], unsigned long long* enc, bool on = true) {
   T m = (T)0;
 #pragma unroll
   for (int t = 0; t < NT; ++t)
 #pragma unroll
     for (int q = 0; q < E; ++q) m = max(m, v[t][q].x * v[t][q].x + v[t][q].y * v[t][q].y);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(enc, enc_ordered((double)m));
+  m = group_max<TPF>(m);
+  if (on && group_first<TPF>()) atomicMax(enc, enc_ordered((double)m));
 }
 
 template <typename T, int N, bool CFL>
@@ -483,7 +480,7 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
     for (int t = 0; t < NR; ++t) v[t][q] = z[t];
   }
   F::template run<+1>(v, lane, sm, tw);
-  if constexpr (CFL) cfl_max_sq<T, NR, C::E>(v, cfl_enc);
+  if constexpr (CFL) cfl_max_sq<T, NR, C::E, C::TPF>(v, cfl_enc);
   // each thread reads back only the positions it wrote: no barrier needed
   auto z1 = [&](int t, int q) -> cpx<T> { return hold[t * N + lane + q * C::TPF]; };
 #pragma unroll
@@ -596,18 +593,7 @@ k_passB_split(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, D
     for (int t = 0; t < NR; ++t) v[t][q] = z[t];
   }
   F::template run<+1>(v, lane, sm, tw);
-  if constexpr (CFL) {  // CFL maximum of |grad psi|^2 from z1 (cfl_max_sq; every lane joins the shuffles)
-    T m = (T)0;
-    if (j == 0) {
-#pragma unroll
-      for (int t = 0; t < NR; ++t)
-#pragma unroll
-        for (int q = 0; q < E; ++q) m = max(m, v[t][q].x * v[t][q].x + v[t][q].y * v[t][q].y);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(cfl_enc, enc_ordered((double)m));
-  }
+  if constexpr (CFL) cfl_max_sq<T, NR, E, TPF>(v, cfl_enc, j == 0);  // of z1: the first group's transform
 #pragma unroll
   for (int t = 0; t < NR; ++t)
 #pragma unroll
@@ -808,7 +794,7 @@ k_passB_pipe(const float2* __restrict__ tf, float2* __restrict__ pb, int kxo, De
       }
       F::template run<+1>(v, lane, sm, tw);
       if (f == 0) {
-        if constexpr (CFL) cfl_max_sq<T, NT, E>(v, cfl_enc);
+        if constexpr (CFL) cfl_max_sq<T, NT, E, TPF>(v, cfl_enc);
         // each thread reads back only the positions it wrote: no barrier needed
 #pragma unroll
         for (int t = 0; t < NT; ++t)

@@ -125,7 +125,7 @@ __device__ __forceinline__ void passB_lean_pair(int rp, float2* tf, float2* __re
     }
     F::template run<+1, true>(v, lane, sm, tw);
     if (f == 0) {
-      if constexpr (CFL) cfl_max_sq<T, 2, E>(v, cfl_enc);
+      if constexpr (CFL) cfl_max_sq<T, 2, E, TPF>(v, cfl_enc);
 #pragma unroll
       for (int q = 0; q < E; ++q) hold[lane + q * TPF] = make_float4(v[0][q].x, v[0][q].y, v[1][q].x, v[1][q].y);
     } else if (f == 1) {

@@ -297,9 +297,8 @@ struct PassB64 {
       }
       m = e == 0x7ff ? 0.0 : scalbn(m, 2 * k);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(enc, enc_ordered(m));
+    m = group_max<TPF>(m);
+    if (on && group_first<TPF>()) atomicMax(enc, enc_ordered(m));
   }
   // a transform's value (held exchanged) in FP64, without its 2^k
   static __device__ __forceinline__ double2 value(fx u) {
