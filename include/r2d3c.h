@@ -24,7 +24,9 @@
  *   - Supported grids: n = 16, 32, ..., 8192 (powers of two).
  *   - Precision: R2D3C_FP64 keeps the fields in FP64 (the drop-in path) and
  *     computes in FP64 but for the transforms, which run in 64-bit block fixed
- *     point (errors below those of FP64 arithmetic);
+ *     point (relative L2 errors at or below those of FP64 arithmetic over noise,
+ *     peaks on noise, power-law spectra and single modes, n = 512 .. 8192:
+ *     0.3 to 0.98 of them);
  *     R2D3C_FP32 keeps the fields and transforms in FP32 (compensated
  *     twiddles) and every diagnostic reduction in FP64.
  */

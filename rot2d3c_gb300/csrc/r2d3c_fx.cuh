@@ -12,15 +12,20 @@
 // min(R_s max|x|, sum|x|) 4^-(s-1): R_s the product of the radices so far,
 // and each twiddle product divides by 4 (the twiddles are scaled by 2^62 and
 // the product keeps the upper 64 bits), which about keeps pace with the
-// growth of a radix-8 stage (sqrt 8 for noise).  The largest of these bounds
-// is scaled to just under 2^62 (the products and the sqrt(1/2) rotations need
-// one more bit).  The rounding noise is about 2.5 units per output, so the
-// relative L2 error of a 4096-point transform is 2^-54 .. 2^-55 for smooth or
-// noisy spectra, against 2^-52 for the same transform in FP64 arithmetic; the
-// two bounds together keep it below FP64's for single modes (sum = max) as
-// for white noise (sum = N mean).  Against long double, a 1024^2 2-D transform
-// (white noise / k^-3 / one mode): 1.1e-16 / 6.7e-17 / 5.9e-17, with FP64
-// arithmetic 3.1e-16 / 2.6e-16 / 3.3e-16.  2048^2 there and back: 548 -> 153 us.
+// growth of a radix-8 stage (sqrt 8 for noise).  It is also at most
+// sqrt(R_1 sum|x|^2), R_1 the first radix (Cauchy and Schwarz over the R_s
+// values that it sums: sqrt(R_s) 4^-(s-1) falls from stage to stage).  The
+// smaller of the last and the largest over the stages of the first two is
+// scaled to just under 2^62 (the products and the sqrt(1/2) rotations need one
+// more bit).  The rounding noise is about 2.5 units per output.  Flat vectors
+// take the first bound, single values the second, a few peaks on noise (the
+// brackets of an intermittent field) the third.
+//   Relative L2 error over that of the same transform in FP64 arithmetic, the
+// worst of noise, its powers, peaks of 5 to 640 on it, power laws and single
+// modes, n = 512 .. 8192: 0.74, 0.64, 0.82, 0.98, 0.89; without the third bound
+// 0.74, 1.18, 1.71, 2.7, 3.3.  A 1024^2 2-D transform against long double (white
+// noise / k^-3 / one mode): 1.1e-16 / 6.7e-17 / 5.9e-17, with FP64 arithmetic
+// 3.1e-16 / 2.6e-16 / 3.3e-16.  2048^2 there and back: 548 -> 156 us.
 #pragma once
 
 #include <vector>
@@ -291,9 +296,10 @@ struct BlockFFT<double, N, E, 1, ILV_OK> {
   // group's, below 32 threads) largest component; every magnitude is then
   // taken relative to it in FP32 (fx_mag), which loses no exponent range; mh
   // becomes the warp's largest word (0: all zero, whatever fx_mag says).
-  // combine: from the thread's largest magnitude mx of a component and the sum
-  // l1 of its values' larger components the group's biased exponent e and the scale s, such that
-  // x 2^(s - (e - 1023)) is the fixed-point value.
+  // combine: from the thread's largest magnitude mx of a component, the sum l1
+  // of its values' larger components and the sum l2 of their squares the group's
+  // biased exponent e and the scale s, such that x 2^(s - (e - 1023)) is the
+  // fixed-point value.
   static constexpr int SUB = TPF < 32 ? TPF : 32;
   static __device__ __forceinline__ int warp_base(unsigned& mh) {
     if constexpr (TPF >= 32) {
@@ -313,72 +319,125 @@ struct BlockFFT<double, N, E, 1, ILV_OK> {
       return m;
     }
   }
-  static __device__ __forceinline__ void combine(int ew, float mx, float l1, int lane, int4* red, int& e, int& s) {
-    mx = sub_max(mx);
+  // The bound by the squares (l2) is taken from four stages on (n >= 1024); with
+  // three the other two leave the error below 0.75 times FP64's.
+  static constexpr bool L2 = NST >= 4;
+  static_assert(!L2 || (TPF >= 64 && E <= 16 && WARPS <= 16), "the ranges of lanes_sum");
+  static __device__ __forceinline__ float shfl_sum(float v, int o0) {
 #pragma unroll
-    for (int o = SUB / 2; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+    for (int o = o0; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+  // 2^LG times the sum of v over the warp, every v to half a unit of 2^-LG (v <=
+  // 2^(23 - LG)): one integer reduction instead of five shuffles and additions.
+  template <int LG>
+  static __device__ __forceinline__ float lanes_sum(float v) {
+    const unsigned u = __reduce_add_sync(0xffffffffu, __float_as_uint(fmaf(v, (float)(1 << LG), 8388608.f)));
+    return (float)(u - 32u * 0x4b000000u);
+  }
+  // 2^-k and 2^k for the exponent k of mx >= 1 (or mx = 0)
+  static __device__ __forceinline__ void unit_of(float mx, float& down, float& up) {
+    up = __int_as_float(__float_as_int(fmaxf(mx, 1.f)) & 0x7f800000);
+    down = __int_as_float((254 << 23) - __float_as_int(up));
+  }
+  static __device__ __forceinline__ void combine(int ew, float mx, float l1, float l2, int lane, int4* red, int& e,
+                                                 int& s) {
+    mx = sub_max(mx);
     e = ew;
+    if constexpr (L2) {
+      // per thread below 2 E and 4 E in units of mx
+      float down, up;
+      unit_of(mx, down, up);
+      l1 = lanes_sum<17>(l1 * down) * (up * 0x1p-17f);
+      l2 = lanes_sum<16>(l2 * down * down) * (up * up * 0x1p-16f);
+    } else {
+      l1 = shfl_sum(l1, SUB / 2);
+    }
     if constexpr (TPF > 32) {
-      if ((lane & 31) == 0) red[lane >> 5] = make_int4(ew, __float_as_int(mx), __float_as_int(l1), 0);
+      if ((lane & 31) == 0)
+        red[lane >> 5] = make_int4(ew, __float_as_int(mx), __float_as_int(l1), __float_as_int(l2));
       __syncthreads();
       const int4 w = red[lane & (WARPS - 1)];
       e = __reduce_max_sync(0xffffffffu, w.x);
       const float f = __int_as_float(max(127 + w.x - e, 0) << 23);
       mx = sub_max(__int_as_float(w.y) * f);
       l1 = __int_as_float(w.z) * f;
-#pragma unroll
-      for (int o = WARPS / 2; o > 0; o >>= 1) l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+      if constexpr (L2) {  // (every warp's entry is read by 32 / WARPS lanes)
+        constexpr float r = (float)WARPS / 32.f;
+        float down, up;
+        unit_of(mx, down, up);
+        l1 = lanes_sum<12>(l1 * down) * (up * 0x1p-12f * r);
+        l2 = lanes_sum<11>(__int_as_float(w.w) * f * f * down * down) * (up * up * 0x1p-11f * r);
+      } else {
+        l1 = shfl_sum(l1, WARPS / 2);
+      }
     }
-    s = scale_of(mx, l1) - (e == 1 ? 2 : 0);  // (subnormals: taken up to twice too small or large)
+    s = scale_of(mx, l1, l2) - (e == 1 ? 2 : 0);  // (subnormals: taken up to twice too small or large)
     if (l1 == 0.f) {  // all zero
       e = 1023;
       s = 0;
     }
   }
   // s for magnitudes relative to the vector's exponent
-  static __device__ __forceinline__ int scale_of(float mx, float l1) {
+  static __device__ __forceinline__ int scale_of(float mx, float l1, float l2) {
     // upper bounds: |z| <= sqrt(2) max(|re|, |im|), the truncated lower words,
-    // the FP32 sums
+    // the FP32 sums (lanes_sum: 2^-12 and 2^-9 of mx, 2^-11 and 2^-8 of mx^2)
     mx *= 1.41423f;
-    l1 *= 1.41425f;
+    l1 *= L2 ? 1.41425f * 1.0025f : 1.41425f;
     float b = 0.f, g = 1.f;
 #pragma unroll
     for (int st = 0; st < NST; ++st) {
       b = fmaxf(b, fminf(mx * (float)ns_of(st + 1), l1) * g);
       g *= 0.25f;
     }
-    return min(62 - ((__float_as_int(b) >> 23) - 126), 61);
+    int x = (__float_as_int(b) >> 23) - 127;  // b < 2^(x + 1)
+    // sqrt(R_s) 4^-(s-1) is largest at the first stage (R <= 16); half the
+    // exponent is the root's
+    if constexpr (L2) x = min(x, ((__float_as_int(l2 * (2.0001f * 1.0046f * (float)E)) >> 23) - 127) >> 1);
+    return min(61 - x, 61);
   }
   // The scale of a vector whose real and imaginary parts are scaled apart, so
   // that the smaller one keeps its own precision: each part relative to its
   // own largest exponent e1, e2 (equal to the other's where it is all zero).
-  // Values 0 or normal; ew and l1 of each part as for combine.
-  static __device__ __forceinline__ void combine2(int ew1, int ew2, float l1, float l2, int lane, int4* red, int& e1,
-                                                  int& e2, int& s) {
-    e1 = ew1;
-    e2 = ew2;
-    float l;
+  // Values 0 or normal; ew, l1 and l2 of each part as for combine (p: part 1,
+  // q: part 2).  Takes two elements of red a warp.
+  static __device__ __forceinline__ void combine2(int ewp, int ewq, float p1, float q1, float p2, float q2, int lane,
+                                                  int4* red, int& e1, int& e2, int& s) {
+    e1 = ewp;
+    e2 = ewq;
+    float l1, l2 = 0.f;
     if constexpr (TPF > 32) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-        l2 += __shfl_xor_sync(0xffffffffu, l2, o);
+      if constexpr (L2) {
+        p1 = lanes_sum<17>(p1);
+        q1 = lanes_sum<17>(q1);
+        p2 = lanes_sum<16>(p2);
+        q2 = lanes_sum<16>(q2);
+      } else {
+        p1 = shfl_sum(p1, 16);
+        q1 = shfl_sum(q1, 16);
       }
-      if ((lane & 31) == 0) red[lane >> 5] = make_int4(ew1, ew2, __float_as_int(l1), __float_as_int(l2));
+      if ((lane & 31) == 0) {
+        red[lane >> 5] = make_int4(ewp, ewq, __float_as_int(p1), __float_as_int(q1));
+        if constexpr (L2) red[WARPS + (lane >> 5)] = make_int4(__float_as_int(p2), __float_as_int(q2), 0, 0);
+      }
       __syncthreads();
       const int4 w = red[lane & (WARPS - 1)];
       e1 = __reduce_max_sync(0xffffffffu, w.x);
       e2 = __reduce_max_sync(0xffffffffu, w.y);
-      l = __int_as_float(w.z) * __int_as_float(max(127 + w.x - e1, 0) << 23) +
-          __int_as_float(w.w) * __int_as_float(max(127 + w.y - e2, 0) << 23);
-#pragma unroll
-      for (int o = WARPS / 2; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+      const float f1 = __int_as_float(max(127 + w.x - e1, 0) << 23), f2 = __int_as_float(max(127 + w.y - e2, 0) << 23);
+      l1 = __int_as_float(w.z) * f1 + __int_as_float(w.w) * f2;
+      if constexpr (L2) {
+        const int4 v = red[WARPS + (lane & (WARPS - 1))];
+        constexpr float r = (float)WARPS / 32.f;
+        l1 = lanes_sum<12>(l1 * 0x1p-17f) * (0x1p-12f * r);
+        l2 = lanes_sum<11>((__int_as_float(v.x) * f1 * f1 + __int_as_float(v.y) * f2 * f2) * 0x1p-16f) * (0x1p-11f * r);
+      } else {
+        l1 = shfl_sum(l1, WARPS / 2);
+      }
     } else {
-      l = l1 + l2;
-#pragma unroll
-      for (int o = SUB / 2; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+      l1 = shfl_sum(p1 + q1, SUB / 2);
     }
-    s = scale_of(2.f, 0.70711f * l);  // (l bounds |z| itself)
+    s = scale_of(2.f, 0.70711f * l1, 0.50001f * l2);  // (the sums are of |z| and |z|^2 themselves)
     if (e1 == 1) e1 = e2 == 1 ? 1023 : e2;
     if (e2 == 1) e2 = e1;
   }
@@ -393,14 +452,15 @@ struct BlockFFT<double, N, E, 1, ILV_OK> {
     }
     mh = fx_any(mh, lo);
     const int ew = warp_base(mh);
-    float mx = 0.f, l1 = 0.f;
+    float mx = 0.f, l1 = 0.f, l2 = 0.f;
 #pragma unroll
     for (int q = 0; q < E; ++q) {
       const float a = fx_mag(max(fx_upper(v[q].x), fx_upper(v[q].y)), ew);
       mx = fmaxf(mx, a);
       l1 += a;
+      l2 = fmaf(a, a, l2);
     }
-    combine(ew, mh ? mx : 0.f, mh ? l1 : 0.f, lane, red, e, s);
+    combine(ew, mh ? mx : 0.f, mh ? l1 : 0.f, mh ? l2 : 0.f, lane, red, e, s);
   }
 
   // Position of value i of one component in a buffer of N 8-byte values

@@ -91,7 +91,7 @@ k_passA64(const double2* __restrict__ ps, const double2* __restrict__ vz, double
     }
     mh = fx_any(mh, lo);
     const int ew = F::warp_base(mh);
-    float mx = 0.f, l1 = 0.f;
+    float mx = 0.f, l1 = 0.f, l2 = 0.f;
 #pragma unroll
     for (int q = 0; q < E; ++q) {
       if (P::dead(q)) continue;
@@ -99,9 +99,10 @@ k_passA64(const double2* __restrict__ ps, const double2* __restrict__ vz, double
       const float a = fx_mag(max(fx_upper(x[q].x), fx_upper(x[q].y)), ew) * __uint2float_ru(absmult(q));
       mx = fmaxf(mx, a);
       l1 += a;
+      l2 = fmaf(a, a, l2);
     }
     int e, s;
-    F::combine(ew, mh ? mx : 0.f, mh ? l1 : 0.f, lane, reinterpret_cast<int4*>(sm + F::RED), e, s);
+    F::combine(ew, mh ? mx : 0.f, mh ? l1 : 0.f, mh ? l2 : 0.f, lane, reinterpret_cast<int4*>(sm + F::RED), e, s);
     const int c = e + 62 - s;
     const bool sub = fx_sub(e);
     fx u[E];
@@ -154,7 +155,7 @@ struct PassB64 {
   // per group: the exchange buffer (mirror slots: re of kx at kx, im at N/2 +
   // 1 + kx), the scale's reduction, z1
   static constexpr size_t XB = (size_t)(N + 8) * 8;
-  static constexpr size_t RED = (size_t)(F::WARPS > 0 ? F::WARPS : 1) * 16;
+  static constexpr size_t RED = (size_t)(F::WARPS > 0 ? F::WARPS : 1) * (F::L2 ? 32 : 16);  // (combine2's)
   static constexpr size_t GROUP = XB + RED + (size_t)N * 16;
   static constexpr int MIRROR = N / 2 + 1;
 
@@ -177,17 +178,19 @@ struct PassB64 {
     }
     mh = fx_any(mh, lo);
     const int ew = F::warp_base(mh);
-    float mx = 0.f, l1 = 0.f;
+    float mx = 0.f, l1 = 0.f, l2 = 0.f;
 #pragma unroll
     for (int q = 0; q < KQ; ++q) {
-      // |Z| <= |A| + |B|
-      const float p = fx_mag(max(fx_upper(a[q].x), fx_upper(a[q].y)), ew) +
-                      fx_mag(max(fx_upper(b[q].x), fx_upper(b[q].y)), ew);
+      // |Z| <= |A| + |B|; |Z[kx]|^2 + |Z[N - kx]|^2 = 2 (|A|^2 + |B|^2)
+      const float ma = fx_mag(max(fx_upper(a[q].x), fx_upper(a[q].y)), ew);
+      const float mb = fx_mag(max(fx_upper(b[q].x), fx_upper(b[q].y)), ew);
+      const float p = ma + mb, w = lane + q * TPF == 0 ? 1.f : 2.f;  // Z[kx] and Z[N - kx]
       mx = fmaxf(mx, p);
-      l1 += lane + q * TPF == 0 ? p : 2.f * p;  // Z[kx] and Z[N - kx]
+      l1 = fmaf(w, p, l1);
+      l2 = fmaf(w, fmaf(ma, ma, mb * mb), l2);
     }
     int s;
-    F::combine(ew, mh ? mx : 0.f, mh ? l1 : 0.f, lane, reinterpret_cast<int4*>(sm + XB), e, s);
+    F::combine(ew, mh ? mx : 0.f, mh ? l1 : 0.f, mh ? l2 : 0.f, lane, reinterpret_cast<int4*>(sm + XB), e, s);
     k = F::out_exp(e, s);
     const int c = e + 62 - s;
     const bool sub = fx_sub(e);
@@ -240,14 +243,18 @@ struct PassB64 {
       m2 = max(m2, fx_upper(p2[q]));
     }
     const int w1 = F::warp_base(m1), w2 = F::warp_base(m2);
-    float l1 = 0.f, l2 = 0.f;
+    float s1 = 0.f, s2 = 0.f, t1 = 0.f, t2 = 0.f;
 #pragma unroll
     for (int q = 0; q < E; ++q) {
-      l1 += fx_mag(fx_upper(p1[q]), w1);
-      l2 += fx_mag(fx_upper(p2[q]), w2);
+      const float a = fx_mag(fx_upper(p1[q]), w1), b = fx_mag(fx_upper(p2[q]), w2);
+      s1 += a;
+      s2 += b;
+      t1 = fmaf(a, a, t1);
+      t2 = fmaf(b, b, t2);
     }
     int e1, e2, s;
-    F::combine2(w1, w2, m1 ? l1 : 0.f, m2 ? l2 : 0.f, lane, reinterpret_cast<int4*>(sm + XB), e1, e2, s);
+    F::combine2(w1, w2, m1 ? s1 : 0.f, m2 ? s2 : 0.f, m1 ? t1 : 0.f, m2 ? t2 : 0.f, lane,
+                reinterpret_cast<int4*>(sm + XB), e1, e2, s);
     const int c1 = e1 + 62 - s, c2 = e2 + 62 - s;
     fx u[E];
 #pragma unroll
