@@ -190,8 +190,6 @@ k_halfplane_sums(const cpx<T>* __restrict__ p0, const cpx<T>* __restrict__ p1,
   for (int t = 0; t < kMaxTerms; ++t) acc[t] = 0.0;
   const cpx<T>* planes[4] = {p0, p1, p2, p3};
   const size_t total = (size_t)gd.nh * gd.n;
-  bool neg = false;
-  for (int k = 0; k < sl.npow; ++k) neg |= sl.kin[k] < 0;
   for (size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x; idx < total;
        idx += (size_t)gridDim.x * blockDim.x) {
     int i, j;
@@ -220,10 +218,10 @@ k_halfplane_sums(const cpx<T>* __restrict__ p0, const cpx<T>* __restrict__ p1,
       const double r = b.x * a.x + b.y * a.y;
       prod[p] = i == 0 ? r : r + r;  // two = 1 on the kx = 0 column
     }
-    const double inv = neg && k2 >= 1 ? 1.0 / ka2 : 0.0;
     for (int k = 0; k < sl.npow; ++k) {
       const int e = sl.kin[k];
-      pw[k] = e == 0 ? 1.0 : e > 0 ? powi(ka2, e) : powi(inv, -e);
+      // (a power of a rounded 1 / ka2 would be off by e units)
+      pw[k] = e == 0 ? 1.0 : e > 0 ? powi(ka2, e) : k2 >= 1 ? recip(powi(ka2, -e)) : 0.0;
     }
     int where = (k2 >= 1 ? W_NONZERO : 0) | (k2 <= gd.kmaxi ? W_DISC : 0);
     if (ka2 <= sl.band_hi && ka2 >= sl.band_lo) where |= W_BAND;

@@ -475,25 +475,6 @@ static __global__ void k_rk_table(double* d1, double* d2, double* ik2, double* w
   }
 }
 
-// 1/d: an FP32 estimate r and one step r (1 + t + t^2), t = 1 - d r, of the
-// hyperpower iteration of third order (M. Altman, Pacific J. Math. 10, 1960),
-// three FP64 operations instead of the division's dozen.  The estimate is of d
-// truncated to 24 bits (2^-23) and one unit off (2^-23), so |t| < 2^-22 and the
-// step leaves t^3 < 2^-66: the nearest double but where 1/d lies that close to a
-// tie, at most 0.5 + 2^-13 units off.  d outside 2^+-100, negative or not finite
-// takes the division.
-__device__ __forceinline__ double recip(double d) {
-  const int hi = __double2hiint(d);
-  if ((unsigned)(hi - ((1023 - 100) << 20)) > (200u << 20)) return 1.0 / d;
-  const float f = __int_as_float(((hi - (896 << 20)) << 3) | (int)((unsigned)__double2loint(d) >> 29));
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
-  const int b = __float_as_int(r);
-  const double r0 = __hiloint2double((b >> 3) + (896 << 20), b << 29);
-  const double t = fma(-d, r0, 1.0);
-  return fma(r0, fma(t, t, t), r0);
-}
-
 // Each CTA transforms one bracket of its columns (blockIdx.z: 0 [psi, -k^2
 // psi], 1 [psi, vz]) and updates the field it drives: C1 needs the first
 // bracket and C2's input, C2 the second and C1's input (see k_passC).

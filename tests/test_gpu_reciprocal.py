@@ -1,4 +1,4 @@
-"""The reciprocal of the FP64 update's divisor (recip, r2d3c_pass64.cuh) against
+"""The reciprocal of the FP64 update's divisor (recip, r2d3c_kernels.cuh) against
 the division, in a small library of its own built from the header.
 
 Tolerance: half a unit in the last place and what the iteration leaves, 2^-66
