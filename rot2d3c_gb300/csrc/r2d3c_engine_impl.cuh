@@ -1489,8 +1489,11 @@ class EngineT final : public IEngine {
         };
         std::vector<CandC> cands;
         for (int g = GB; g >= 1; g /= 2) {
+          if constexpr (kLeanC<T, N>) {  // one shape: a group per CTA, two CTAs per column pair
+            cands.push_back({0, 1, 2, 1});
+            break;
+          }
           cands.push_back({0, g, 1, 1});
-          if constexpr (kLeanC<T, N>) break;  // its launch shape is fixed
           if constexpr (kChunkC<T, N>) {
             cands.push_back({0, g, 2, 1});
             // teams of 2 or 4 groups per column pair share its update
@@ -1609,9 +1612,9 @@ class EngineT final : public IEngine {
       if (forced[0] > GAr) throw Error(kEINVAL, "R2D3C_GROUPS: more pass-A groups per CTA than its radix allows");
       ga_ = forced[0] >= 0 ? (forced[0] ? forced[0] : GAr) : tune_a_[ka].mode;
       fa_ = forced[1] >= 0 ? forced[1] : tune_a_[ka].grid;
-      auto pick_bc = [&](const std::vector<TuneRec>& t, const char* env, const char* pair_name, int forced_g,
+      auto pick_bc = [&](const std::vector<TuneRec>& t, const char* env, const char* pair_name, int full, int forced_g,
                          int& mode, int& grid, int& groups) {
-        auto ok = [&](const TuneRec& r) { return pol == 0 || r.mode == 1 || (r.mode == 0 && r.grid == GB); };
+        auto ok = [&](const TuneRec& r) { return pol == 0 || r.mode == 1 || (r.mode == 0 && r.grid == full); };
         const size_t pick0 = argmin(t, [&](const TuneRec& r) { return r.mode == 0 && ok(r); });
         size_t pick = argmin(t, ok);
         if (pol == 2) {  // the persistent form wherever it exists
@@ -1644,8 +1647,9 @@ class EngineT final : public IEngine {
         groups = forced_g >= 0 ? (forced_g ? forced_g : GB) : t[pick0].grid;
         return pick0;
       };
-      pick_bc(tune_, "R2D3C_PASSB", "per_row_pair", forced[2], passb_mode_, pipeb_grid_, gb_);
-      const size_t c0 = pick_bc(tune_c_, "R2D3C_PASSC", "per_column_pair", forced[3], passc_mode_, pipec_grid_, gc_);
+      pick_bc(tune_, "R2D3C_PASSB", "per_row_pair", GB, forced[2], passb_mode_, pipeb_grid_, gb_);
+      const size_t c0 = pick_bc(tune_c_, "R2D3C_PASSC", "per_column_pair", kLeanC<T, N> ? 1 : GB, forced[3],
+                                passc_mode_, pipec_grid_, gc_);
       fc_ = forced[4] > 0 ? forced[4] : (c0 < tune_c_.size() ? tune_c_[c0].chunks : 1);
       // a forced pass-C group count without a forced team width runs one group per column pair
       wc_ = forced[5] > 0 ? forced[5] : forced[3] >= 0 ? 1 : (c0 < tune_c_.size() ? tune_c_[c0].wide : 1);
@@ -1664,6 +1668,10 @@ class EngineT final : public IEngine {
           }
       }
       if (wc_ > gc_) throw Error(kEINVAL, "R2D3C_GROUPS: pass C team wider than its groups per CTA");
+      if constexpr (kLeanC<T, N>) {  // the shape that runs, whatever was asked for
+        gc_ = wc_ = 1;
+        fc_ = 2;
+      }
     });
   }
   void set_plan_policy(int policy) override {
@@ -1706,16 +1714,25 @@ class EngineT final : public IEngine {
                  tune_c_[i].grid, (double)tune_c_[i].us);
       else
         snprintf(b, sizeof b,
-                 "%s{\"variant\": \"per_column_pair\", \"groups\": %d, \"chunks\": %d, \"team\": %d, \"us\": %.2f}",
+                 "%s{\"variant\": \"per_column_pair\", \"groups\": %d, \"chunks\": %d, \"team\": %d, \"us\": %.2f",
                  i ? ", " : "", tune_c_[i].grid, tune_c_[i].chunks, tune_c_[i].wide, (double)tune_c_[i].us);
       r += b;
+      if (!tune_c_[i].mode) {
+        b[0] = 0;
+        if (tune_c_[i].us_fused > 0.f) snprintf(b, sizeof b, ", \"us_with_a\": %.2f", (double)tune_c_[i].us_fused);
+        r += std::string(b) + "}";
+      }
     }
     snprintf(b, sizeof b,
              "], \"chosen_c\": \"%s\", \"ctas_c\": %d, \"groups_c\": %d, \"chunks_c\": %d, \"team_c\": %d, "
-             "\"fused_ca\": %s}",
+             "\"fused_ca\": %s",
              passc_mode_ ? "persistent" : "per_column_pair", passc_mode_ == 1 ? pipec_grid_ : 0, gc_, fc_, wc_,
              fuse_ca() ? "true" : "false");
-    return r + b;
+    r += b;
+    b[0] = 0;
+    if (fuse_ca())  // the shape of pass C with the next substep's pass A
+      snprintf(b, sizeof b, ", \"groups_ca\": %d, \"chunks_ca\": %d, \"team_ca\": %d", gf_, ff_, wf_);
+    return r + b + "}";
   }
 
  private:
