@@ -37,6 +37,11 @@ def test_shape_of_pass_c_with_pass_a(gpu, monkeypatch, n):
     rep = _report(gpu, n)
     assert rep["fused_ca"]
     timed = [r for r in rep["pass_c"] if "us_with_a" in r]
+    # only shapes near the fastest without it are timed with it: creating a context pays for each
+    pairs = [r for r in rep["pass_c"] if r["variant"] == "per_column_pair"]
+    near = 1.15 * min(r["us"] for r in pairs)
+    assert all(("us_with_a" in r) == (r["us"] <= near) for r in pairs if abs(r["us"] - near) > 0.02)
+    assert len(timed) < len(pairs)
     best = min(timed, key=lambda r: r["us_with_a"])
     chosen = [r for r in timed
               if (r["groups"], r["chunks"], r["team"]) == (rep["groups_ca"], rep["chunks_ca"], rep["team_ca"])]
