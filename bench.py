@@ -316,9 +316,16 @@ def pass_flops(n):
     return {"A": 6 * M * per, "B": 4 * n * per, "C": 2 * M * per}
 
 
+def pass_tag(n, real_bytes):
+    """Which passes run at this size: "fp64", "fp32_lean" (FP32 from n = 2048:
+    k_passB_lean, and k_passC_lean) or "fp32"."""
+    return "fp64" if real_bytes == 8 else "fp32_lean" if n >= 2048 else "fp32"
+
+
 def pass_traffic(n, tag, top):
     """DRAM bytes (read + write) per launch of pass `top` from the committed
-    ncu summary profiles/pass_traffic_<tag>_n<n>.json, or None."""
+    ncu summary profiles/pass_traffic_<tag>_n<n>.json, or None, and which
+    kernel of which file they are."""
     path = os.path.join(ROOT, "profiles", f"pass_traffic_{tag}_n{n}.json")
     if not os.path.exists(path):
         return None, None
@@ -326,7 +333,7 @@ def pass_traffic(n, tag, top):
         tr = json.load(f).get(f"k_pass{top}")
     if not tr:
         return None, None
-    return tr["dram_read"] + tr["dram_write"], os.path.relpath(path, ROOT) + " (ncu)"
+    return tr["dram_read"] + tr["dram_write"], os.path.relpath(path, ROOT) + f" (ncu, {tr['kernel']})"
 
 
 def roofline_of(ms, cnt, n, real_bytes, tag, hbm, peak_kind, peak64=None):
@@ -350,7 +357,8 @@ def roofline_of(ms, cnt, n, real_bytes, tag, hbm, peak_kind, peak64=None):
     top = max("ABC", key=lambda k: passes[k]["ms_per_launch"])
     ach = passes[top]["achieved_gbs"]
     traffic, tsrc = pass_traffic(n, tag, top)
-    r = {"bound": "hbm", "kernel": f"k_pass{top}{'64' if real_bytes == 8 else ''} ({'FP64' if real_bytes == 8 else 'FP32'}, n={n})",
+    form = "64" if real_bytes == 8 else "_lean" if tag == "fp32_lean" and top != "A" else ""
+    r = {"bound": "hbm", "kernel": f"k_pass{top}{form} ({'FP64' if real_bytes == 8 else 'FP32'}, n={n})",
          "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": peak_kind,
          "traffic": traffic, "traffic_source": tsrc, "algorithmic_bytes_per_launch": pb[top], "passes": passes}
     if peak64:
@@ -826,7 +834,7 @@ def main():
         clocks = clk.summary()
         ms64, cnt64 = c64.profile_passes(min(K, 4), dt)
         peak64 = R.fp64_fma_peak()
-        roofline = roofline_of(ms64, cnt64, n, 8, "fp64", hbm, peak_kind, peak64)
+        roofline = roofline_of(ms64, cnt64, n, 8, pass_tag(n, 8), hbm, peak_kind, peak64)
         e2e = e2e_roundtrip(c64, ps, vz, dt, min(K, args.e2e_steps), torch, world)
         e2e_loop = e2e_main_loop(c64, ps, vz, args.loop_steps, torch, world) if args.loop_steps > 0 else None
         plan64 = plan_summary(c64)
@@ -846,7 +854,7 @@ def main():
         fp32 = {"value": v32, "unit": UNIT, "ms_per_step": 1e3 * el32 / K32, "steps": K32,
                 "dtype": "f32 (compensated twiddles, FP64 reductions)",
                 "fp32_speedup": v32 / v64 if v64 else None, "gpu_launches": launches32,
-                "roofline": roofline_of(ms32, cnt32, n, 4, "fp32", hbm, peak_kind),
+                "roofline": roofline_of(ms32, cnt32, n, 4, pass_tag(n, 4), hbm, peak_kind),
                 "e2e": e2e_roundtrip(c32, ps, vz, dt, min(K32, 50), torch, world),
                 "clocks": clk32.summary(), "plan": plan_summary(c32)}
         if s64 is not None:

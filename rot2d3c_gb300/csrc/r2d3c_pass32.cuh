@@ -5,7 +5,7 @@
 // CTA) and now: B 60 / 247 / 2660 -> 57 / 234 / 1216, C 36 / 137 / 394 -> 29 /
 // 102 / 490 (the 8192^2 C pays for the pair-tiled layout that its B takes).
 // B waits on its loads (planes and twiddles: 61 KB of (hi, lo) pairs a
-// 4096-point transform, of which L1 keeps a fifth) and issues in 46% of the
+// 4096-point transform, of which L1 keeps a fifth) and issues in 51% of the
 // slots; C on its update's loads, DRAM 41% of peak.
 //   Tried for B: radix 8 with 64 registers and 32 warps an SM (262 us), most of
 // z1 in global memory so that L1 holds the twiddles (268).  For C: the shared

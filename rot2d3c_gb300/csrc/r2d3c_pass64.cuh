@@ -6,7 +6,7 @@
 // Per launch at 4096^2 (us; FP64 arithmetic, the transforms alone in fixed
 // point, these kernels): A 2556, 841, 381; B 5227, 1697, 942; C 1179, 594,
 // 270.  What bounds them now (ncu): A and B the issue of integer instructions
-// (50-55% of the slots, ALU pipe 54-55%), C the FP64 pipe of the update (70%)
+// (52-57% of the slots, ALU pipe 55-56%), C the FP64 pipe of the update (70%)
 // and the latency of its loads; DRAM 11-33% of peak.
 #pragma once
 
