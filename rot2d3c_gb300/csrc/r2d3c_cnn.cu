@@ -113,13 +113,6 @@ __device__ __forceinline__ void ldsm_x4_t(unsigned (&r)[4], const void* p) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(a));
 }
-__device__ __forceinline__ void ldsm_x2_t(unsigned (&r)[2], const void* p) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
-  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
-               : "=r"(r[0]), "=r"(r[1])
-               : "r"(a));
-}
-
 // Halo tile (TH+2) x (TW+2) pixels of CIN channels around tile (b, ty0, tx0),
 // periodic wrap, into the swizzled layout.
 template <int CIN>

@@ -1047,13 +1047,12 @@ class EngineT final : public IEngine {
     });
   }
   // forward y-FFT of the nh columns of a product plane in the passes' mixed
-  // layout (pair-tiled in the FP32 tiled mode)
+  // (pair-tiled) layout
   void launch_colfft_mixed(const cpx<T>* in, cpx<T>* out) {
     dispatch_n(n_, [&](auto NC) {
       constexpr int N = decltype(NC)::value;
-      constexpr int PY = sizeof(T) == 8 ? 2 : PassNT<T, N>::value;
       using C = Cfg<T, N>;
-      auto k = k_colfft<T, N, -1, PY>;
+      auto k = k_colfft<T, N, -1, 2>;
       const int g = fft_groups(gd_.nh, C::G);
       k<<<(gd_.nh + g - 1) / g, C::TPF * g, g * C::FFT::SMEM_BYTES, st_>>>(in, out, gd_.nh, tw_, gd_.nh, nullptr,
                                                                                    0x7fffffff);
@@ -1134,10 +1133,12 @@ class EngineT final : public IEngine {
     }
     const int g = gb_ ? gb_ : Cfg<T, N>::G;  // groups per CTA: autotuned
     const dim3 grid((N + g - 1) / g, nb);
-    if (kxo > gd_.M)
-      k_passB64<N, CFL, true><<<grid, B::TPF * g, g * B::GROUP, st_>>>(tf, pb, kxo, gd_, tw_, enc_base_, batch());
-    else
+    if (kxo > gd_.M) {
+      if constexpr (CFL) throw Error(kESTATE, "pass B: the CFL maximum comes with the retained columns only");
+      else k_passB64<N, false, true><<<grid, B::TPF * g, g * B::GROUP, st_>>>(tf, pb, kxo, gd_, tw_, enc_base_, batch());
+    } else {
       k_passB64<N, CFL, false><<<grid, B::TPF * g, g * B::GROUP, st_>>>(tf, pb, kxo, gd_, tw_, enc_base_, batch());
+    }
     post("k_passB64");
   }
   // (FP64, and FP32 from n = 2048: the derivative planes are used up)
@@ -1160,8 +1161,10 @@ class EngineT final : public IEngine {
         const tw_t<T>* tw = PassAE<T, N>::value == L::E ? tw_a_ : tw_;
         static_assert(PassAE<T, N>::value == L::E || Cfg<T, N>::E == L::E, "pass B radix has a twiddle table");
         if (kxo > gd_.M) {
-          k_passB_lean<N, CFL, true, false><<<dim3(N / 2, nb), L::TPF, L::SMEM, st_>>>(tf, pb, kxo, gd_, inv4, tw,
-                                                                                       enc_base_, batch());
+          if constexpr (CFL) throw Error(kESTATE, "pass B: the CFL maximum comes with the retained columns only");
+          else
+            k_passB_lean<N, false, true, false><<<dim3(N / 2, nb), L::TPF, L::SMEM, st_>>>(tf, pb, kxo, gd_, inv4, tw,
+                                                                                           enc_base_, batch());
         } else if (passb_mode_ == 1) {
           // persistent: the autotuned CTA count (about as many as fit at once)
           const int per_run = std::max(1, std::min(N / 2, (pipeb_grid_ + nb - 1) / nb));
@@ -1268,7 +1271,7 @@ class EngineT final : public IEngine {
       constexpr size_t sm = Cfg<T, N>::SMEM;
       set_smem_attr(k_colfft<T, N, -1>, sm);
       set_smem_attr(k_colfft<T, N, +1>, sm);
-      set_smem_attr(k_colfft<T, N, -1, sizeof(T) == 8 ? 2 : PassNT<T, N>::value>, sm);
+      set_smem_attr(k_colfft<T, N, -1, 2>, sm);
       set_smem_attr(k_rowc2r<T, N>, sm);
       set_smem_attr(k_rowr2c<T, N>, sm);
       set_smem_attr(k_cnn2_to_rows<T, N>, sm);

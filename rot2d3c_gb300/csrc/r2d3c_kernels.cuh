@@ -315,7 +315,7 @@ k_rowr2c(const T* __restrict__ rin, cpx<T>* __restrict__ tout, const tw_t<T>* __
 // both as 16-byte column pairs of the pair-tiled plane.
 // --------------------------------------------------------------------------
 template <typename T, int N, int EA = PassAE<T, N>::value>
-__global__ void __launch_bounds__(CfgAE<T, N, EA>::THREADS, (sizeof(T) == 4 && CfgAE<T, N, EA>::THREADS == 256) ? 2 : 1)
+__global__ void __launch_bounds__(CfgAE<T, N, EA>::THREADS, CfgAE<T, N, EA>::THREADS == 256 ? 2 : 1)
 k_passA(const cpx<T>* __restrict__ ps, const cpx<T>* __restrict__ vz, cpx<T>* __restrict__ tf,
         DevGrid gd, const tw_t<T>* __restrict__ tw, Batch bs) {
   constexpr int NT = PassNT<T, N>::value;
@@ -367,56 +367,37 @@ k_passA(const cpx<T>* __restrict__ ps, const cpx<T>* __restrict__ vz, cpx<T>* __
       }
       F::template run<+1>(v, lane, sm, tw);
       cpx<T>* dst = tf + (size_t)f * plane;
-      if constexpr (NT == 2) {
-        // lanes (2p, 2p+1) hold rows y = 2p, 2p+1 of columns kx0, kx0+1: swap
-        // one value so each lane writes one column's row pair (16 bytes)
-        const bool odd = lane & 1;
-        const int kx = kx0 + (odd ? 1 : 0);
+      static_assert(NT == 2, "column pairs");
+      // lanes (2p, 2p+1) hold rows y = 2p, 2p+1 of columns kx0, kx0+1: swap
+      // one value so each lane writes one column's row pair (16 bytes)
+      const bool odd = lane & 1;
+      const int kx = kx0 + (odd ? 1 : 0);
 #pragma unroll
-        for (int q = 0; q < C::E; ++q) {
-          const cpx<T> give = odd ? v[0][q] : v[1][q];
-          cpx<T> got;
-          got.x = __shfl_xor_sync(0xffffffffu, give.x, 1);
-          got.y = __shfl_xor_sync(0xffffffffu, give.y, 1);
-          const int y = (lane + q * C::TPF) & ~1;
-          if (kx < gd.M) {
-            const cpx<T> lo = odd ? got : v[0][q];
-            const cpx<T> hi = odd ? v[1][q] : got;
-            *reinterpret_cast<float4*>(dst + mix_idx<N, 2>(kx, y, gd.M)) = make_float4(lo.x, lo.y, hi.x, hi.y);
-          }
-        }
-      } else {
-        if (kx0 < gd.M) {
-#pragma unroll
-          for (int q = 0; q < C::E; ++q) dst[(size_t)kx0 * N + lane + q * C::TPF] = v[0][q];
+      for (int q = 0; q < C::E; ++q) {
+        const cpx<T> give = odd ? v[0][q] : v[1][q];
+        cpx<T> got;
+        got.x = __shfl_xor_sync(0xffffffffu, give.x, 1);
+        got.y = __shfl_xor_sync(0xffffffffu, give.y, 1);
+        const int y = (lane + q * C::TPF) & ~1;
+        if (kx < gd.M) {
+          const cpx<T> lo = odd ? got : v[0][q];
+          const cpx<T> hi = odd ? v[1][q] : got;
+          *reinterpret_cast<float4*>(dst + mix_idx<N, 2>(kx, y, gd.M)) = make_float4(lo.x, lo.y, hi.x, hi.y);
         }
       }
     }
   }
 }
 
-// NR consecutive rows y0.. of a mixed plane at column kx: one 16-byte load
-// for two FP32 rows.
-template <typename T, int NR>
-__device__ __forceinline__ void load_rows(const cpx<T>* __restrict__ p, size_t off, cpx<T> (&o)[NR]) {
-  if constexpr (NR == 2 && sizeof(T) == 4) {
-    const float4 w = __ldg(reinterpret_cast<const float4*>(p + off));
-    o[0] = mkc<T>(w.x, w.y);
-    o[1] = mkc<T>(w.z, w.w);
-  } else {
-#pragma unroll
-    for (int t = 0; t < NR; ++t) o[t] = p[off + t];
-  }
+// Two consecutive rows y0, y0 + 1 of a mixed plane at column kx: one 16-byte
+// access.
+__device__ __forceinline__ void load_rows(const float2* __restrict__ p, size_t off, float2 (&o)[2]) {
+  const float4 w = __ldg(reinterpret_cast<const float4*>(p + off));
+  o[0] = make_float2(w.x, w.y);
+  o[1] = make_float2(w.z, w.w);
 }
-
-template <typename T, int NR>
-__device__ __forceinline__ void store_rows(cpx<T>* __restrict__ p, size_t off, const cpx<T> (&o)[NR]) {
-  if constexpr (NR == 2 && sizeof(T) == 4) {
-    *reinterpret_cast<float4*>(p + off) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
-  } else {
-#pragma unroll
-    for (int t = 0; t < NR; ++t) p[off + t] = o[t];
-  }
+__device__ __forceinline__ void store_rows(float2* __restrict__ p, size_t off, const float2 (&o)[2]) {
+  *reinterpret_cast<float4*>(p + off) = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
 }
 
 // Packed spectrum of a pair of mixed planes (A, B) at rows y0.. for x-position
@@ -428,8 +409,8 @@ __device__ __forceinline__ void packed_pair(const cpx<T>* __restrict__ pa, const
     const int kk = k < M ? k : N - k;
     cpx<T> a[NR], b[NR];
     const size_t off = mix_idx<N, NR>(kk, y0, M);
-    load_rows<T, NR>(pa, off, a);
-    load_rows<T, NR>(pb, off, b);
+    load_rows(pa, off, a);
+    load_rows(pb, off, b);
 #pragma unroll
     for (int t = 0; t < NR; ++t) {
       if (k == 0) {
@@ -557,8 +538,8 @@ k_passB(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, DevGrid
         o2[t] = mkc<T>((w.y + u.y) * h, (u.x - w.x) * h);
       }
       const size_t off = mix_idx<N, NR>(k, y0, gd.nh);
-      store_rows<T, NR>(pb, off, o1);
-      store_rows<T, NR>(pb + oplane, off, o2);
+      store_rows(pb, off, o1);
+      store_rows(pb + oplane, off, o2);
     }
   }
 }
@@ -649,8 +630,8 @@ k_passB_split(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, D
         o2[t] = mkc<T>((w.y + u.y) * h, (u.x - w.x) * h);
       }
       const size_t off = mix_idx<N, NR>(k, y0, gd.nh);
-      store_rows<T, NR>(pb, off, o1);
-      store_rows<T, NR>(pb + oplane, off, o2);
+      store_rows(pb, off, o1);
+      store_rows(pb + oplane, off, o2);
     }
   }
 }
@@ -858,13 +839,8 @@ k_passB_pipe(const float2* __restrict__ tf, float2* __restrict__ pb, int kxo, De
           o2[t] = mkc<T>((w.y + u.y) * h, (u.x - w.x) * h);
         }
         const size_t off = mix_idx<N, 2>(k, y0 + r0, gd.nh);
-        if constexpr (NT == 2) {
-          store_rows<T, 2>(pb, off, o1);
-          store_rows<T, 2>(pb + oplane, off, o2);
-        } else {
-          pb[off] = o1[0];
-          pb[oplane + off] = o2[0];
-        }
+        store_rows(pb, off, o1);
+        store_rows(pb + oplane, off, o2);
       }
     }
   }
@@ -1128,31 +1104,26 @@ k_passC(const cpx<T>* __restrict__ pb, const cpx<T>* c1in, const cpx<T>* c2in,
     // hoisted out of the loop and held in registers across it
     const int lane = opaque(lane0);
     const cpx<T>* src = pb + pl * oplane;
-    if constexpr (NT == 2) {
-      // lane pair (2p, 2p+1): the even lane loads column kx0's rows (2p, 2p+1),
-      // the odd lane column kx0+1's; one swap gives each lane its own row of
-      // both columns
-      const bool odd = lane & 1;
-      const int kx = kx0 + (odd ? 1 : 0);
+    static_assert(NT == 2, "column pairs");
+    // lane pair (2p, 2p+1): the even lane loads column kx0's rows (2p, 2p+1),
+    // the odd lane column kx0+1's; one swap gives each lane its own row of
+    // both columns
+    const bool odd = lane & 1;
+    const int kx = kx0 + (odd ? 1 : 0);
 #pragma unroll
-      for (int q = 0; q < C::E; ++q) {
-        const int y = (lane + q * C::TPF) & ~1;
-        const float4 w = __ldg(reinterpret_cast<const float4*>(src + mix_idx<N, 2>(kx, y, gd.nh)));
-        const float gx = odd ? w.x : w.z, gy = odd ? w.y : w.w;  // value the partner needs
-        const float rx = __shfl_xor_sync(0xffffffffu, gx, 1);
-        const float ry = __shfl_xor_sync(0xffffffffu, gy, 1);
-        if (odd) {
-          v[0][q] = mkc<T>(rx, ry);
-          v[1][q] = mkc<T>(w.z, w.w);
-        } else {
-          v[0][q] = mkc<T>(w.x, w.y);
-          v[1][q] = mkc<T>(rx, ry);
-        }
+    for (int q = 0; q < C::E; ++q) {
+      const int y = (lane + q * C::TPF) & ~1;
+      const float4 w = __ldg(reinterpret_cast<const float4*>(src + mix_idx<N, 2>(kx, y, gd.nh)));
+      const float gx = odd ? w.x : w.z, gy = odd ? w.y : w.w;  // value the partner needs
+      const float rx = __shfl_xor_sync(0xffffffffu, gx, 1);
+      const float ry = __shfl_xor_sync(0xffffffffu, gy, 1);
+      if (odd) {
+        v[0][q] = mkc<T>(rx, ry);
+        v[1][q] = mkc<T>(w.z, w.w);
+      } else {
+        v[0][q] = mkc<T>(w.x, w.y);
+        v[1][q] = mkc<T>(rx, ry);
       }
-    } else {
-      const cpx<T>* s5 = src + (size_t)(kx0 < gd.M ? kx0 : 0) * N;
-#pragma unroll
-      for (int q = 0; q < C::E; ++q) v[0][q] = s5[lane + q * C::TPF];
     }
     F::template run<-1>(v, lane, sm, tw);
     if (pl == 0) {

@@ -174,8 +174,8 @@ __device__ __forceinline__ void passB_lean_pair(int rp, float2* tf, float2* __re
         o2[t] = mkc<T>((w.y + u.y) * h, (u.x - w.x) * h);
       }
       const size_t off = mix_idx<N, 2>(k, 2 * rp, gd.nh);
-      store_rows<T, 2>(pb, off, o1);
-      store_rows<T, 2>(pb + oplane, off, o2);
+      store_rows(pb, off, o1);
+      store_rows(pb + oplane, off, o2);
     }
   }
 }
