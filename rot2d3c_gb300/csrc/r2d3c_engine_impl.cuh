@@ -1371,10 +1371,12 @@ class EngineT final : public IEngine {
   // and the fastest of each pass is kept:
   //   A: transform groups per CTA (the config's G down to 1) x field chunks
   //      (the six fields in 1, 2, 3 or 6 CTAs);
-  //   B: one group per row pair, G down to 1 groups per CTA, or (n = 512 ..
-  //      4096 FP32) persistent cp.async-staged CTAs, as many as are resident
-  //      or half of that;
-  //   C: the same with column pairs.
+  //   B: one group per row pair, G down to 1 groups per CTA, or (FP32 from n =
+  //      512 on) persistent CTAs, staged by cp.async below n = 2048, as many
+  //      as are resident or half of that, or (small grids) split;
+  //   C: the same with column pairs (persistent and staged for FP32 n = 512 ..
+  //      4096; not split, but in chunks and teams, and one lean shape from n =
+  //      1024 on).
   // Small grids gain from spreading the work over more SMs (256^2: the
   // config's groups fill 6 CTAs in pass A); large ones from full CTAs.
   // Pass A's radix (FP32, n = 1024 .. 4096) is chosen as FFTW's measured
@@ -1634,7 +1636,7 @@ class EngineT final : public IEngine {
           if (pp < t.size()) pick = pp;
         }
         // env=<pair_name>|persistent overrides the measured choice
-        // (persistent where it exists: FP32, n = 512 .. 4096)
+        // (persistent where it exists: FP32, pass B from n = 512 on, C 512 .. 4096)
         if (const char* force = std::getenv(env)) {
           if (std::strcmp(force, pair_name) == 0) {
             pick = pick0;

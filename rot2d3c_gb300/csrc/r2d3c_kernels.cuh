@@ -637,8 +637,8 @@ k_passB_split(const cpx<T>* __restrict__ tf, cpx<T>* __restrict__ pb, int kxo, D
 }
 
 // --------------------------------------------------------------------------
-// Pass B, FP32 pair-tiled grids (n = 512 .. 4096), one row pair per CTA at a
-// time: persistent CTAs that stage each row pair's mixed-plane inputs in
+// Pass B, FP32 grids n = 512 and 1024 (above: k_passB_lean), one row pair per CTA
+// at a time: persistent CTAs that stage each row pair's mixed-plane inputs in
 // shared memory with asynchronous copies (cp.async, 16 bytes per thread and
 // instruction) one plane pair ahead of the transform that needs it, so that
 // the global loads of pairs 2 and 3 and of the next row pair's pair 1 overlap
